@@ -164,7 +164,7 @@ void Workspace::release() {
     DevBuf *all[] = {&X, &C0, &Cout, &labels, &d2, &xnorm, &Ccur, &Cnew, &Ct, &h, &queue, &H, &Gs,
                      &counts, &offsets, &piece_base, &perm, &records, &shift_part, &shift_tiles, &empty_flag,
                      &empty_ids,
-                     &sel_hist, &sel_state, &cand, &obj_part, &scalars, &state, &Xhi, &Xlo, &Chi, &Clo, &tcx, &rowb, &pp_acc, &pp_rand,
+                     &sel_state, &cand, &obj_part, &scalars, &state, &Xhi, &Xlo, &Chi, &Clo, &tcx, &rowb, &pp_acc, &pp_rand,
                      &pp_state, &pp_flags, &csr_vals, &csr_cols64, &csr_rowptr64, &csr_cols, &csr_rowptr,
                      &csr_bad, &csr_cnorm, &ex_acc, &ex_cnt, &ex_prev, &ex_colexp, &ex_records};
     for (DevBuf *b : all) {
@@ -279,8 +279,13 @@ int ensure_common(kmb_context *ctx, int64_t n, int64_t d, int64_t k, bool rechec
     return KMB_OK;
 }
 
-__global__ void reset_iteration_kernel(LoopState *st) {
+// Before a pass: its counters, and max ||c|| (the previous pass's kept in *cmax_prev
+// when given).
+__global__ void reset_iteration_kernel(LoopState *st, double *cmax, double *cmax_prev) {
     if (st->done) return;
+    if (cmax_prev) *cmax_prev = *cmax;
+    *cmax = 0.0;
+    st->n_empty = 0;
     st->n_recheck = 0;
     st->n_changed = 0;
     st->n_full = 0;
@@ -305,10 +310,9 @@ int assign_pass_tc<float>(kmb_context *ctx, const float *X, int64_t n, int64_t d
     kmb::Workspace &ws = ctx->ws;
     cudaStream_t s = ctx->stream;
     kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    reset_iteration_kernel<<<1, 1, 0, s>>>(st);
+    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, &sc->cnorm_max_prev);
     KMB_LAUNCHED();
-    kmb::launch_prep_centroids_tc(C, k, d, ws.Chi.ptr, ws.Clo.ptr, (float *)ws.h.ptr, &sc->cnorm_max,
-                                  &sc->cnorm_max_prev, st, s);
+    kmb::launch_prep_centroids_tc(C, k, d, ws.Chi.ptr, ws.Clo.ptr, (float *)ws.h.ptr, &sc->cnorm_max, st, s);
     int rc;
     {
         KernelTimer timer(ctx, 1);
@@ -342,7 +346,7 @@ int assign_pass(kmb_context *ctx, const F *X, int64_t n, int64_t d, const F *C, 
     cudaStream_t s = ctx->stream;
     const int64_t kpad = round_up(k, kBN);
     kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    reset_iteration_kernel<<<1, 1, 0, s>>>(st);
+    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, nullptr);
     KMB_LAUNCHED();
     kmb::launch_prep_centroids<F>(C, k, d, kpad, (F *)ws.Ct.ptr, (F *)ws.h.ptr, &sc->cnorm_max, st, s);
     {
@@ -431,11 +435,13 @@ void init_state(LoopState &h, double eps) {
 // cluster sums, moved rows only once few rows move), double rows the FP64 one.
 template <typename F>
 int prepare_update(kmb_context *ctx, const F *X, int64_t n, int64_t d, int64_t k, LoopState *st) {
+    kmb::prepare_update_tail(ctx->ws, ctx->stream);
     return KMB_OK;
 }
 template <>
 int prepare_update<float>(kmb_context *ctx, const float *X, int64_t n, int64_t d, int64_t k, LoopState *st) {
     if (!kmb::ensure_exact_buffers(ctx->ws, n, k, d)) return fail(ctx, KMB_ENOMEM, "exact update buffers");
+    kmb::prepare_update_tail(ctx->ws, ctx->stream);
     kmb::prepare_exact_update(X, n, d, ctx->ws, st, ctx->stream);
     return KMB_OK;
 }
@@ -777,7 +783,7 @@ void csr_assign_pass(kmb_context *ctx, const kmb::CsrRows &X, const F *C, int64_
     cudaStream_t s = ctx->stream;
     const int64_t kpad = round_up(k, kBN);
     kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    reset_iteration_kernel<<<1, 1, 0, s>>>(st);
+    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, nullptr);
     KMB_LAUNCHED();
     kmb::launch_prep_centroids<F>(C, k, X.d, kpad, (F *)ws.Ct.ptr, (F *)ws.h.ptr, &sc->cnorm_max, st, s);
     KernelTimer timer(ctx, 0);
@@ -838,7 +844,10 @@ int train_csr_impl(kmb_context *ctx, int memory, const void *vals, const int64_t
     KMB_CUDA(cudaMemsetAsync(sc, 0, sizeof(kmb::DevScalars), s));
     KMB_CUDA(cudaMemcpyAsync(Ccur, C0, sizeof(F) * k * d, cudaMemcpyDeviceToDevice, s));
     const int64_t T = p->max_iteration_count;
-    if (T > 0) csr_prepare_update<F>(X, ws, st, s);
+    if (T > 0) {
+        kmb::prepare_update_tail(ws, s);
+        csr_prepare_update<F>(X, ws, st, s);
+    }
     int64_t enq = 0, batch = 2;
     while (enq < T) {
         const int64_t upto = std::min(T, enq + batch);

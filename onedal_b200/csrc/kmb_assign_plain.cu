@@ -354,11 +354,6 @@ __global__ void row_norms_kernel(const F *__restrict__ X, int64_t n, int d, F *_
     }
 }
 
-__global__ void reset_double_kernel(double *p, const LoopState *st) {
-    if (st && st->done) return;
-    *p = 0.0;
-}
-
 constexpr int kSmallK = 32;        // clusters handled by assign_small_kernel
 constexpr int kSmallThreads = 128;
 
@@ -801,8 +796,6 @@ template <typename F>
 void launch_prep_centroids(const F *C, int64_t k, int64_t d, int64_t kpad, F *Ct, F *h, double *cnorm_max,
                            const LoopState *st, cudaStream_t s) {
     const int dpad = (int)((d + BK - 1) / BK * BK);
-    reset_double_kernel<<<1, 1, 0, s>>>(cnorm_max, st);
-    KMB_LAUNCHED();
     prep_centroids_kernel<F><<<(unsigned)kpad, 128, 0, s>>>(C, (int)k, (int)d, dpad, (int)kpad, Ct, h, cnorm_max, st);
     KMB_LAUNCHED();
 }

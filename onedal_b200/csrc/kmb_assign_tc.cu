@@ -953,12 +953,6 @@ __global__ void prep_centroids_tc_kernel(const float *__restrict__ C, int k, int
     }
 }
 
-__global__ void reset_cmax_kernel(double *p, double *prev, const LoopState *st) {
-    if (st && st->done) return;
-    *prev = *p;
-    *p = 0.0;
-}
-
 }  // namespace tc
 
 // Hand-off slots are indexed by %smid (a CTA needs a whole SM's shared memory,
@@ -991,10 +985,8 @@ void launch_split_rows(const float *X, int64_t rows, int64_t d, void *hi, void *
 }
 
 void launch_prep_centroids_tc(const float *C, int64_t k, int64_t d, void *Chi, void *Clo, float *h, double *cnorm_max,
-                              double *cnorm_max_prev, const LoopState *st, cudaStream_t s) {
+                              const LoopState *st, cudaStream_t s) {
     const int64_t dpad = tc_dpad(d), kpad = tc_kpad(k);
-    tc::reset_cmax_kernel<<<1, 1, 0, s>>>(cnorm_max, cnorm_max_prev, st);
-    KMB_LAUNCHED();
     tc::prep_centroids_tc_kernel<<<(unsigned)kpad, 128, 0, s>>>(C, (int)k, (int)d, (int)dpad, (int)kpad,
                                                                  (__nv_bfloat16 *)Chi, (__nv_bfloat16 *)Clo, h,
                                                                  cnorm_max, st);

@@ -118,7 +118,7 @@ struct Workspace {
     cudaStream_t stream = nullptr;
     DevBuf X, C0, Cout, labels, d2, xnorm, Ccur, Cnew, Ct, h, queue;
     DevBuf H, Gs, counts, offsets, piece_base, perm, records, shift_part, shift_tiles, empty_flag, empty_ids;
-    DevBuf sel_hist, sel_state, cand, obj_part, scalars, state;
+    DevBuf sel_state, cand, obj_part, scalars, state;
     DevBuf Xhi, Xlo, Chi, Clo, tcx, rowb, pp_acc, pp_rand, pp_state, pp_flags;
     DevBuf csr_vals, csr_cols64, csr_rowptr64, csr_cols, csr_rowptr, csr_bad, csr_cnorm;
     DevBuf ex_acc, ex_cnt, ex_prev, ex_colexp, ex_records;  // exact update: limb sums, counts, previous
@@ -141,7 +141,8 @@ struct DevScalars {
 
 // ---- assignment (plain FMA form) ------------------------------------------
 // Prepares per-iteration centroid data: transposed copy Ct (d x kpad), half
-// squared norms h (kpad, +inf padding) and max ||c|| for the error bound.
+// squared norms h (kpad, +inf padding) and max ||c|| for the error bound (the caller
+// has cleared *cnorm_max).
 template <typename F>
 void launch_prep_centroids(const F *C, int64_t k, int64_t d, int64_t kpad, F *Ct, F *h, double *cnorm_max,
                            const LoopState *st, cudaStream_t s);
@@ -175,10 +176,10 @@ bool tc_supported(int64_t d); // dpad <= 256
 // same value launch_row_norms gives).
 void launch_split_rows(const float *X, int64_t rows, int64_t d, void *hi, void *lo, float *xnorm, int num_sms,
                        cudaStream_t s);
-// C -> Chi/Clo [kpad][dpad], -h = -0.5||c||^2 (kpad, -inf padding), max ||c||.
-// Also moves the previous max ||c|| into *cnorm_max_prev before recomputing it.
+// C -> Chi/Clo [kpad][dpad], -h = -0.5||c||^2 (kpad, -inf padding), max ||c|| (the
+// caller has cleared *cnorm_max).
 void launch_prep_centroids_tc(const float *C, int64_t k, int64_t d, void *Chi, void *Clo, float *h,
-                              double *cnorm_max, double *cnorm_max_prev, const LoopState *st, cudaStream_t s);
+                              double *cnorm_max, const LoopState *st, cudaStream_t s);
 // xchg: tc_xchg_bytes(num_sms) bytes of device scratch (epilogue hand-off).
 // prior: labels/d2 hold the previous pass's results under the centroids that
 // the update in between moved by sqrt(shift_part[j]); they seed a lower bound
@@ -232,6 +233,9 @@ UpdatePlan make_update_plan(int64_t n, int64_t k, int64_t d);
 // Sizes the update buffers of `ws` for plan `p` (false on allocation failure).
 // fp64_records false: no FP64 piece records (an update that never sums pieces in FP64).
 bool ensure_update_buffers(Workspace &ws, const UpdatePlan &p, size_t fsize, bool fp64_records = true);
+// Clears the state that an update's kernels share (barrier, tickets): once per call,
+// before its first update.
+void prepare_update_tail(Workspace &ws, cudaStream_t s);
 
 // One Lloyd update: counting-sort the rows by label (stable, so each cluster's
 // rows are summed in row order), FP64 sums per fixed piece of rows, centroid =

@@ -146,9 +146,10 @@ int infer_noalloc(const F *X, int64_t n, int64_t d, const F *C, int64_t k, int32
     p += align256(sizeof(F) * kpad);
     double *partials = (double *)p;
     p += align256(sizeof(double) * kObjectivePartials);
-    double *cnorm_max = (double *)p;  // zeroed by the centroid preparation on every call
+    double *cnorm_max = (double *)p;  // cleared on every call
 
     launch_row_norms<F>(X, n, d, xnorm, s);
+    cudaMemsetAsync(cnorm_max, 0, sizeof(double), s);
     launch_prep_centroids<F>(C, k, d, kpad, Ct, h, cnorm_max, nullptr, s);
     launch_assign_plain<F>(X, n, d, Ct, h, k, kpad, xnorm, cnorm_max, labels, d2, nullptr, nullptr, s);
     if (objective) launch_objective<F>(X, n, d, C, labels, partials, objective, s);

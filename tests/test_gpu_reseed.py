@@ -1,0 +1,46 @@
+"""Empty clusters take the rows with the largest squared distances, (distance descending,
+row ascending): the grid-wide selection at its edges -- one candidate, as many as rows
+allow, more than the shared-memory sort holds, ties at the threshold that only some rows
+of may be taken, one CTA and many. Coordinates are small integers, so distances are exact
+in either type and the expected rows are known without a tolerance."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from onedal_b200 import _native
+
+pytestmark = pytest.mark.gpu
+
+
+def _step(X, C):
+    ctx = _native.context(0)
+    n, d = X.shape
+    Xd, Cd = torch.from_numpy(X).cuda(), torch.from_numpy(C).cuda()
+    out, lab = torch.empty_like(Cd), torch.empty(n, dtype=torch.int32, device="cuda")
+    shift, ne = ctypes.c_double(), ctypes.c_int64()
+    ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+    dtype = _native.KMB_F32 if X.dtype == np.float32 else _native.KMB_F64
+    ctx.check(ctx.lib.kmb_lloyd_step(ctx.handle, dtype, Xd.data_ptr(), n, d, Cd.data_ptr(), C.shape[0],
+                                     _native.KMB_FORM_PLAIN, 0, out.data_ptr(), lab.data_ptr(), ctypes.byref(shift),
+                                     ctypes.byref(ne)))
+    return out.cpu().numpy(), lab.cpu().numpy(), ne.value
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n,m,span", [(2, 1, 9), (40, 39, 2), (5000, 1, 4), (5000, 512, 2), (5000, 1024, 40),
+                                      (5000, 1025, 3), (4097, 7, 1), (700_001, 300, 3), (700_001, 3, 300)])
+def test_empty_clusters_take_the_farthest_rows(dt, n, m, span):
+    d = 3
+    rng = np.random.default_rng(n + m)
+    X = rng.integers(-span, span + 1, (n, d)).astype(dt)
+    if span == 1:
+        X[:] = 1  # every distance equal: the lowest rows
+    C = np.zeros((m + 1, d), dt)
+    C[1:] = 10000.0  # nobody's nearest
+    out, lab, ne = _step(X, C)
+    assert ne == m and (lab == 0).all()
+    dist = (X.astype(np.int64) ** 2).sum(1)
+    order = np.lexsort((np.arange(n), -dist))[:m]
+    np.testing.assert_array_equal(out[1:], X[order])
