@@ -422,32 +422,58 @@ __device__ __forceinline__ void top3_insert(Top3 &r, float &thr, float thr0, flo
     thr = ins ? fmaxf(fmaxf(thr0, r.t), __fsub_rd(r.b, band_up)) : thr;
 }
 
-// One 32-column chunk of a row into its running top-3. The chunk is reduced to
-// its maximum (3-input max.f32); only when a lane of the warp holds a value at or
-// above its threshold are the column triples walked, group by group, a triple
-// being visited (warp-uniformly, static register indices) when some lane's
-// triple maximum reaches that lane's threshold.
+// One 32-column chunk of a row into its running top-3. The chunk is reduced to its
+// maximum m1 (3-input max.f32); nothing else happens when no lane's m1 reaches its
+// threshold. Otherwise every lane forms the bit mask of its columns at or above
+// max(threshold, m1 - band) -- one packed subtraction per two columns and one funnel
+// shift of the sign per column, no branches. A column below m1 - band can be neither
+// the row's best nor inside the best's band, so it cannot change the outputs. Nearly
+// always each mask holds m1's column alone, and one insertion of (m1, column) does;
+// when some lane holds several (a near tie inside the chunk), or NaN columns, the
+// column triples are walked in order, a triple being visited (warp-uniformly, static
+// register indices) when some lane's triple maximum reaches that lane's threshold.
+// The epilogue bounded the kernel with a walk of triples for every candidate (32 rows
+// share a warp, so four chunks of five hold some lane's best): 4M x 128, k = 1024, 3.19 ms
+// a launch with the walk alone, 2.36 ms with the mask; 1M x 20, k = 1000, 476 and 370 us.
 __device__ __forceinline__ void scan_chunk(const float (&w)[32], int colbase, float thr0, float band_up, float &thr,
                                            Top3 &r) {
     float m[11];
 #pragma unroll
     for (int i = 0; i < 10; ++i) m[i] = max3f(w[3 * i], w[3 * i + 1], w[3 * i + 2]);
     m[10] = fmaxf(w[30], w[31]);
-    // four groups of triples (columns 0-8, 9-17, 18-26, 27-31): a group is walked
-    // only when some lane's group maximum reaches that lane's threshold
     const float gm[4] = {max3f(m[0], m[1], m[2]), max3f(m[3], m[4], m[5]), max3f(m[6], m[7], m[8]), fmaxf(m[9], m[10])};
     const float m1 = max3f(gm[0], gm[1], fmaxf(gm[2], gm[3]));
-    if (__any_sync(0xffffffffu, m1 >= thr)) {
+    const bool hit = m1 >= thr;
+    if (!__any_sync(0xffffffffu, hit)) return;
+    const float cut = fmaxf(thr, __fsub_rd(m1, band_up));
+    const float2 neg = make_float2(-cut, -cut);
+    unsigned part[4];  // bit i of part[q]: column 8q + i lies below the cut (the sign of w - cut)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (__any_sync(0xffffffffu, gm[q] >= thr)) {
+    for (int q = 0; q < 4; ++q) {
+        unsigned below = 0;
 #pragma unroll
-                for (int g = 3 * q; g < 3 * q + 3 && g < 11; ++g) {
-                    if (__any_sync(0xffffffffu, m[g] >= thr)) {
+        for (int i = 8 * q + 6; i >= 8 * q; i -= 2) {
+            const float2 d = __fadd2_rn(make_float2(w[i], w[i + 1]), neg);
+            below = __funnelshift_l(__float_as_uint(d.y), below, 1);
+            below = __funnelshift_l(__float_as_uint(d.x), below, 1);
+        }
+        part[q] = below;
+    }
+    const unsigned below = __byte_perm(__byte_perm(part[0], part[1], 0x0040), __byte_perm(part[2], part[3], 0x0040), 0x5410);
+    const unsigned in = hit ? ~below : 0u;
+    if (!__any_sync(0xffffffffu, (in & (in - 1u)) != 0u)) {
+        top3_insert(r, thr, thr0, band_up, m1, colbase + __ffs(in) - 1);  // (lanes without a hit insert nothing)
+        return;
+    }
 #pragma unroll
-                        for (int i = 0; i < 3; ++i)
-                            if (3 * g + i < 32) top3_insert(r, thr, thr0, band_up, w[3 * g + i], colbase + 3 * g + i);
-                    }
+    for (int q = 0; q < 4; ++q) {
+        if (__any_sync(0xffffffffu, gm[q] >= thr)) {
+#pragma unroll
+            for (int g = 3 * q; g < 3 * q + 3 && g < 11; ++g) {
+                if (__any_sync(0xffffffffu, m[g] >= thr)) {
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+                        if (3 * g + i < 32) top3_insert(r, thr, thr0, band_up, w[3 * g + i], colbase + 3 * g + i);
                 }
             }
         }
@@ -851,6 +877,289 @@ assign_tc_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_constant
     }
 }
 
+// ---- one cluster tile -------------------------------------------------------
+// All clusters in one tile (k <= BN) and two or more A stages: the same roles, pipeline
+// and arithmetic as assign_tc_kernel, but an epilogue group owns whole row tiles (group
+// g the CTA's tiles g, g + 2, ...) and its own accumulators (slots g, g + 2, ... of the
+// 512 / BN), so a row's top-3 is complete in one thread: no hand-off between groups, no
+// named barrier and no merge per tile, and the centroid panels stay in shared memory for
+// the whole launch when they fit the ring (`resident`: every shape but dpad = 128 at
+// BN = 256 with three products).
+// Bound by the row panels' HBM reads (768 MB at 3M x 50). With the columns of
+// every accumulator split between the groups the hand-off, about 1300 cycles per tile and
+// extra group, bounded it: 3M x 50, k = 20, three products, 317 us a launch, 195 us here.
+// With several cluster tiles the split is the better one (a group's drain of a whole
+// accumulator is then longer than the MMAs of the other group's: 1M x 20, k = 1000,
+// 431 us owned, 373 us split; 20M x 128, k = 1024, 13.1 and 12.1 ms).
+// 32-column chunks that hold only padding are neither read nor refilled; a chunk is read
+// while the previous one is scanned, and the accumulator is released before its last
+// chunk is scanned.
+struct OwnBarriers {
+    uint64_t a_full[4], a_empty[4];
+    uint64_t b_full[MAX_B_STAGES], b_empty[MAX_B_STAGES];
+    uint64_t acc_full[kMaxAcc], acc_empty[kMaxAcc];
+    uint64_t mma_done;
+    uint32_t tmem_base;
+    int abort;
+};
+
+template <int BN, int NPROD>
+__global__ void __launch_bounds__(NTHREADS, 1)
+assign_tc_own_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_constant__ CUtensorMap tmXl,
+                     const __grid_constant__ CUtensorMap tmCh, const __grid_constant__ CUtensorMap tmCl, Params p) {
+    constexpr int NACC = TMEM_COLS / BN;
+    constexpr int NSLOT = NACC / 2;  // accumulators of one group
+    constexpr int PANEL_B = panel_b_bytes(BN);
+    constexpr int KPB = kpb_of(BN);
+    constexpr uint32_t kIdesc = make_idesc(BN);
+    constexpr int NSPLIT = NPROD == 3 ? 2 : 1;
+    constexpr int BSTAGE = NSPLIT * PANEL_B;
+    static_assert(NPROD == 1 || NPROD == 3, "products per k-step");
+    static_assert(NACC >= 2 && NACC <= kMaxAcc && NGROUPS == 2, "accumulators per group");
+    __shared__ int s_skip;  // one read of the loop flag for the whole CTA
+    if (threadIdx.x == 0) s_skip = p.st->done;
+    __syncthreads();
+    if (s_skip) return;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+    const int a_stage_bytes = NSPLIT * p.kpanels * PANEL;
+    uint8_t *A = smem;
+    uint8_t *B = A + (size_t)p.a_stages * a_stage_bytes;
+    OwnBarriers *bar = (OwnBarriers *)(B + (size_t)p.b_stages * BSTAGE);
+    volatile int *abort = &bar->abort;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < p.a_stages; ++i) {
+            mbar_init(&bar->a_full[i], 1);
+            mbar_init(&bar->a_empty[i], 1);
+        }
+        for (int i = 0; i < p.b_stages; ++i) {
+            mbar_init(&bar->b_full[i], 1);
+            mbar_init(&bar->b_empty[i], 1);
+        }
+        for (int i = 0; i < NACC; ++i) {
+            mbar_init(&bar->acc_full[i], 1);
+            mbar_init(&bar->acc_empty[i], 4);  // the owning group's warps
+        }
+        mbar_init(&bar->mma_done, 1);
+        bar->abort = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(su32(&bar->tmem_base)),
+                     "r"(TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem_base = bar->tmem_base;
+    const int unit0 = (int)blockIdx.x, unit_stride = (int)gridDim.x;
+    const int my_tiles = (p.n_tiles - unit0 + unit_stride - 1) / unit_stride;
+    const int nkb = p.kpanels * (KP / KPB);    // B stages of the cluster tile
+    const bool resident = nkb <= p.b_stages;  // B stays
+
+    if (warp == 0) {
+        if (lane == 0) {
+            // ---------------- TMA producer ----------------
+            int a_issued[4] = {0, 0, 0, 0};
+            int b_issued[MAX_B_STAGES];
+            for (int i = 0; i < MAX_B_STAGES; ++i) b_issued[i] = 0;
+            int bs = 0;
+            uint32_t bphase = 0;
+            bool ok = true;
+            for (int lt = 0; lt < my_tiles && ok; ++lt) {
+                const int as = lt & (p.a_stages - 1), ause = lt / p.a_stages;
+                if (!mbar_wait(&bar->a_empty[as], (ause & 1) ^ 1, abort, p.wait_cycles)) { ok = false; break; }
+                mbar_expect_tx(&bar->a_full[as], (uint32_t)a_stage_bytes);
+                uint8_t *Ab = A + (size_t)as * a_stage_bytes;
+                const int row0 = (unit0 + lt * unit_stride) * BM;
+                for (int kp = 0; kp < p.kpanels; ++kp) {
+                    tma_load_2d(Ab + (size_t)kp * PANEL, &tmXh, &bar->a_full[as], kp * KP, row0);
+                    if (NPROD == 3)
+                        tma_load_2d(Ab + (size_t)(p.kpanels + kp) * PANEL, &tmXl, &bar->a_full[as], kp * KP, row0);
+                }
+                a_issued[as]++;
+                if (resident && lt > 0) continue;
+                for (int kb = 0; kb < nkb; ++kb) {
+                    if (!mbar_wait(&bar->b_empty[bs], bphase ^ 1, abort, p.wait_cycles)) { ok = false; break; }
+                    mbar_expect_tx(&bar->b_full[bs], BSTAGE);
+                    uint8_t *Bb = B + (size_t)bs * BSTAGE;
+                    tma_load_2d(Bb, &tmCh, &bar->b_full[bs], kb * KPB, 0);
+                    if (NPROD == 3) tma_load_2d(Bb + PANEL_B, &tmCl, &bar->b_full[bs], kb * KPB, 0);
+                    b_issued[bs]++;
+                    if (++bs == p.b_stages) {
+                        bs = 0;
+                        bphase ^= 1;
+                    }
+                }
+            }
+            if (!ok) {  // do not leave while bulk copies may still land in shared memory
+                for (int i = 0; i < 4; ++i)
+                    if (a_issued[i]) mbar_drain(&bar->a_full[i], (a_issued[i] - 1) & 1);
+                for (int i = 0; i < p.b_stages; ++i)
+                    if (b_issued[i]) mbar_drain(&bar->b_full[i], (b_issued[i] - 1) & 1);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // ---------------- MMA issuer ----------------
+            int bs = 0;
+            uint32_t bphase = 0;
+            bool ok = true;
+            for (int lt = 0; lt < my_tiles && ok; ++lt) {
+                const int as = lt & (p.a_stages - 1), ause = lt / p.a_stages;
+                if (!mbar_wait(&bar->a_full[as], ause & 1, abort, p.wait_cycles)) break;
+                const int own = lt >> 1;  // the owning group's tiles before this one
+                const int slot = (lt & 1) + 2 * (own % NSLOT), use = own / NSLOT;
+                // the owning group has written -h into this accumulator (first use included)
+                if (!mbar_wait(&bar->acc_empty[slot], use & 1, abort, p.wait_cycles)) break;
+                tc_fence_after();
+                const uint32_t a_base = su32(A + (size_t)as * a_stage_bytes);
+                const uint32_t tmem_d = tmem_base + (uint32_t)(slot * BN);
+                if (resident) {
+                    bs = 0;
+                    bphase = 0;
+                }
+                for (int kb = 0; kb < nkb; ++kb) {
+                    if (!mbar_wait(&bar->b_full[bs], bphase, abort, p.wait_cycles)) { ok = false; break; }
+                    tc_fence_after();
+                    const int kp = kb / (KP / KPB), ka = (kb % (KP / KPB)) * (KPB * 2 / 16);
+                    const uint64_t ah = sw128_desc(a_base + kp * PANEL) + ka;
+                    const uint64_t al = sw128_desc(a_base + (p.kpanels + kp) * PANEL) + ka;
+                    const uint64_t bh = swb_desc<KPB>(su32(B + (size_t)bs * BSTAGE));
+                    const uint64_t bl = swb_desc<KPB>(su32(B + (size_t)bs * BSTAGE + PANEL_B));
+#pragma unroll
+                    for (int ks = 0; ks < KPB / 16; ++ks) {
+                        if (NPROD == 1)
+                            mma_bf16x1(tmem_d, ah + 2 * ks, bh + 2 * ks, kIdesc);
+                        else
+                            mma_bf16x3(tmem_d, ah + 2 * ks, al + 2 * ks, bh + 2 * ks, bl + 2 * ks, kIdesc);
+                    }
+                    if (!resident) mma_commit(&bar->b_empty[bs]);
+                    if (++bs == p.b_stages) {
+                        bs = 0;
+                        bphase ^= 1;
+                    }
+                }
+                if (ok) {
+                    mma_commit(&bar->acc_full[slot]);
+                    mma_commit(&bar->a_empty[as]);
+                }
+            }
+            mma_commit(&bar->mma_done);  // all issued MMAs complete before TMEM is released
+            mbar_drain(&bar->mma_done, 0);
+        }
+    } else {
+        // ---------------- epilogue ----------------
+        const int quarter = warp & 3;       // TMEM lanes 32*quarter .. +31
+        const int group = (warp - 2) >> 2;  // 0: warps 2-5, 1: warps 6-9
+        const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16);
+        const int nch = (p.k + 31) >> 5;    // 32-column chunks that hold clusters
+        bool ok = true;
+        for (int a0 = 0; a0 < NSLOT; ++a0) {  // first uses of this group's accumulators
+            const int slot = group + 2 * a0;
+#pragma unroll 1
+            for (int c = 0; c < nch; ++c) {
+                __syncwarp();
+                tmem_st32_from(lane_base + (uint32_t)(slot * BN + 32 * c), p.h + 32 * c);
+            }
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&bar->acc_empty[slot]);
+        }
+        auto row_of = [&](int lt_) { return (int64_t)(unit0 + lt_ * unit_stride) * BM + quarter * 32 + lane; };
+        float2 nb = make_float2(__int_as_float(0xff800000), 0.0f);
+        float nxn = 0.0f;
+        if (group < my_tiles && row_of(group) < p.n) {
+            nb = p.rowb[row_of(group)];
+            nxn = p.xnorm[row_of(group)];
+        }
+        int own = 0;
+        for (int lt = group; lt < my_tiles && ok; lt += 2, ++own) {
+            const int64_t row = row_of(lt);
+            const float thr0 = nb.x, band_up = nb.y;
+            const float xn = nxn;
+            if (lt + 2 < my_tiles && row_of(lt + 2) < p.n) {
+                nb = p.rowb[row_of(lt + 2)];
+                nxn = p.xnorm[row_of(lt + 2)];
+            }
+            Top3 r;  // in y = -score space: b >= s >= t
+            r.b = r.s = r.t = __int_as_float(0xff800000);
+            r.ib = r.is = 0;
+            float thr = thr0;
+            const int slot = group + 2 * (own % NSLOT), use = own / NSLOT;
+            if (!__all_sync(0xffffffffu, mbar_wait(&bar->acc_full[slot], use & 1, abort, p.wait_cycles))) {
+                ok = false;
+                break;
+            }
+            tc_fence_after();
+            const uint32_t taddr = lane_base + (uint32_t)(slot * BN);
+            auto release = [&]() {  // every chunk is read and refilled with -h
+                tmem_wait_st();
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&bar->acc_empty[slot]);
+            };
+            float va[32], vb[32];
+            uint32_t hr[32];
+            __syncwarp();
+            tmem_ld32_nowait(taddr, va);
+#pragma unroll 1
+            for (int c = 0; c < nch; c += 2) {
+                load_h32(p.h + 32 * c, hr);
+                tmem_wait_ld_regs(va);
+                tmem_st32_regs(taddr + 32 * c, hr);
+                if (c + 1 < nch)
+                    tmem_ld32_nowait(taddr + 32 * (c + 1), vb);
+                else
+                    release();
+                scan_chunk(va, 32 * c, thr0, band_up, thr, r);
+                __syncwarp();
+                if (c + 1 < nch) {
+                    load_h32(p.h + 32 * (c + 1), hr);
+                    tmem_wait_ld_regs(vb);
+                    tmem_st32_regs(taddr + 32 * (c + 1), hr);
+                    if (c + 2 < nch)
+                        tmem_ld32_nowait(taddr + 32 * (c + 2), va);
+                    else
+                        release();
+                    scan_chunk(vb, 32 * (c + 1), thr0, band_up, thr, r);
+                    __syncwarp();
+                }
+            }
+            if (row < p.n) {  // back to score space (score = -y)
+                const float b = -r.b;
+                p.labels[row] = r.ib;
+                p.d2[row] = 2.0f * b + xn;
+                if (p.queue) {
+                    // (a row for which no cluster passed the filters -- impossible while the prior
+                    // bound holds -- goes to the full FP64 rescan)
+                    const bool none = !(b < __int_as_float(0x7f800000));
+                    const double bd = (double)b, band = (double)band_up;
+                    if ((double)-r.s - bd <= band || none)
+                        enqueue_recheck(p.queue, p.n, p.st, (int)row, r.ib, r.is, (double)-r.t - bd <= band || none);
+                }
+            }
+        }
+    }
+
+    __syncwarp();
+    tc_fence_before();
+    __syncthreads();
+    if (bar->abort && threadIdx.x == 0) {
+        p.st->error = KMB_ETIMEDOUT;
+        p.st->done = 1;
+    }
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS)
+                     : "memory");
+    }
+}
+
 // Per row, ahead of the tensor-core pass (after the centroid prep has computed
 // max ||c||): the recheck band 2e rounded up, and the prior threshold.
 //   e = 1.0625 ((3.03 u_b^2 + 2 * 3 dpad * 2u) ||x|| cmax + 2u (cmax^2 / 2 + ||x|| cmax))
@@ -1071,11 +1380,15 @@ int launch_assign_tc(const void *Xhi, const void *Xlo, int64_t n, int64_t d, con
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const int kpanels = (int)(dpad / tc::KP);
     const int a_stage = nsplit * kpanels * tc::PANEL;
-    const int fixed = 1024 + (int)sizeof(tc::Barriers) + 64;
+    const int fixed = 1024 + (int)std::max(sizeof(tc::Barriers), sizeof(tc::OwnBarriers)) + 64;
     const int bn = tc_tile_n(k);  // cluster tile (UMMA N); kpad is a multiple of it
     const bool pair = use_cta_pairs();
     const int panel_b = tc::panel_b_bytes(bn, pair);
     int a_stages = (2 * a_stage + 3 * nsplit * panel_b + fixed <= optin) ? 2 : 1;
+    // one cluster tile, on a GPU of its own (a grid of one CTA per row tile has no second
+    // tile to alternate with)
+    const bool own = !pair && a_stages == 2 && kpad == bn && num_sms > 0;
+    if (own && 4 * a_stage + 3 * nsplit * panel_b + fixed <= optin) a_stages = 4;
     int b_stages = (optin - fixed - a_stages * a_stage) / (nsplit * panel_b);
     b_stages = std::min(b_stages, tc::MAX_B_STAGES);
     if (b_stages < 2) return KMB_EUNSUPPORTED;
@@ -1125,6 +1438,16 @@ int launch_assign_tc(const void *Xhi, const void *Xlo, int64_t n, int64_t d, con
         tc::row_bounds_kernel<<<bs, 256, 0, s>>>(n, xnorm, labels, d2, shift_part, cnorm_max, cnorm_max_prev, (int)dpad,
                                                  (int)k, prior ? 1 : 0, products, (float2 *)rowb, st);
         KMB_LAUNCHED();
+    }
+    if (own) {
+        auto kern = products == 1 ? (bn == 256 ? tc::assign_tc_own_kernel<256, 1> : tc::assign_tc_own_kernel<128, 1>)
+                                  : (bn == 256 ? tc::assign_tc_own_kernel<256, 3> : tc::assign_tc_own_kernel<128, 3>);
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+            return KMB_ECUDA;
+        const int grid = num_sms < 0 ? p.n_tiles : (int)std::min<int64_t>(num_sms, p.n_tiles);
+        kern<<<grid, tc::NTHREADS, smem, s>>>(mXh, mXl, mCh, mCl, p);
+        KMB_LAUNCHED();
+        return cudaGetLastError() == cudaSuccess ? KMB_OK : KMB_ECUDA;
     }
     if (!pair) {
         auto kern = products == 1 ? (bn == 256 ? tc::assign_tc_kernel<256, false, 1> : tc::assign_tc_kernel<128, false, 1>)
