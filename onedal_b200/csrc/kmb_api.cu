@@ -136,6 +136,11 @@ cudaMemPool_t library_pool(int dev) {
     return pool;
 }
 
+std::mutex &cooperative_mutex() {
+    static std::mutex mu;
+    return mu;
+}
+
 // From the library's pool when it exists, else the device's default pool.
 cudaError_t pool_alloc(void **p, size_t bytes, int dev, cudaStream_t s) {
     cudaMemPool_t pool = library_pool(dev);
@@ -166,7 +171,7 @@ void Workspace::release() {
                      &empty_ids,
                      &sel_state, &cand, &obj_part, &scalars, &state, &Xhi, &Xlo, &Chi, &Clo, &tcx, &rowb, &pp_acc, &pp_rand,
                      &pp_state, &pp_flags, &csr_vals, &csr_cols64, &csr_rowptr64, &csr_cols, &csr_rowptr,
-                     &csr_bad, &csr_cnorm, &ex_acc, &ex_cnt, &ex_prev, &ex_colexp, &ex_records};
+                     &csr_bad, &csr_cnorm, &small, &ex_acc, &ex_cnt, &ex_prev, &ex_colexp, &ex_records};
     for (DevBuf *b : all) {
         if (b->ptr) cudaFreeAsync(b->ptr, stream);
         b->ptr = nullptr;
@@ -499,6 +504,31 @@ int run_loop(kmb_context *ctx, const F *X, int64_t n, int64_t d, F *C, const kmb
     return KMB_OK;
 }
 
+// A small problem's train (or its iterations only) in one launch; waits for it and leaves
+// its state in h_state[0]. The lock is taken for the launch's whole time on the device.
+template <typename F>
+int run_small(kmb_context *ctx, const kmb::SmallPlan &plan, const F *X, int64_t n, int64_t d, const F *C0,
+              const kmb_params *p, bool final_pass, F *C_out, int32_t *labels) {
+    kmb::Workspace &ws = ctx->ws;
+    cudaStream_t s = ctx->stream;
+    static_assert(sizeof(kmb::SmallOut) <= 2 * sizeof(LoopState), "h_state receives a SmallOut");
+    if (!ws.ensure(ws.small, kmb::small_scratch_bytes<F>(plan, d, p->cluster_count)))
+        return fail(ctx, KMB_ENOMEM, "device allocation failed (n=%lld d=%lld k=%lld)", (long long)n, (long long)d,
+                    (long long)p->cluster_count);
+    ProfRange range("kmb_small_train");
+    std::lock_guard<std::mutex> lock(kmb::cooperative_mutex());
+    {
+        KernelTimer timer(ctx, 0);
+        KMB_CUDA(kmb::launch_small_train<F>(plan, X, n, d, C0, p->cluster_count, p->max_iteration_count,
+                                            p->accuracy_threshold, final_pass, C_out, labels, ws.small.ptr, s));
+    }
+    KMB_CUDA(cudaMemcpyAsync(ctx->h_state, ws.small.ptr, sizeof(kmb::SmallOut), cudaMemcpyDeviceToHost, s));
+    KMB_CUDA(cudaStreamSynchronize(s));
+    if (reinterpret_cast<const kmb::SmallOut *>(ctx->h_state)->sync.error)
+        return fail(ctx, KMB_ETIMEDOUT, "device loop failed (status %d)", KMB_ETIMEDOUT);
+    return KMB_OK;
+}
+
 template <typename F>
 int iterate_impl(kmb_context *ctx, const void *Xv, int64_t n, int64_t d, void *Cv, const kmb_params *p,
                  int32_t *labels, int64_t *iteration_count, kmb_stats *stats) {
@@ -507,6 +537,19 @@ int iterate_impl(kmb_context *ctx, const void *Xv, int64_t n, int64_t d, void *C
     ctx->tc_products = form_products(p->form);
     if (tc && !kmb::tc_supported(d)) return fail(ctx, KMB_EUNSUPPORTED, "tensor-core form needs d <= 256");
     const bool recheck = p->recheck != 0 || tc;
+    const kmb::SmallPlan small = recheck ? kmb::SmallPlan() : kmb::make_small_plan<F>(n, d, k);
+    if (small.ctas) {
+        int rc = run_small<F>(ctx, small, (const F *)Xv, n, d, (const F *)Cv, p, false, (F *)Cv, labels);
+        if (rc) return rc;
+        const LoopState &hs = ctx->h_state[0];
+        if (iteration_count) *iteration_count = hs.iterations;
+        if (stats) {
+            *stats = kmb_stats();
+            stats->empty_cluster_events = hs.empty_events;
+            stats->last_shift = hs.shift;
+        }
+        return KMB_OK;
+    }
     int rc = ensure_common<F>(ctx, n, d, k, recheck, tc);
     if (rc) return rc;
     kmb::UpdatePlan plan = kmb::make_update_plan(n, k, d);
@@ -537,10 +580,14 @@ int train_impl(kmb_context *ctx, int memory, const void *Xv, int64_t n, int64_t 
     ctx->tc_products = form_products(p->form);
     if (tc && !kmb::tc_supported(d)) return fail(ctx, KMB_EUNSUPPORTED, "tensor-core form needs d <= 256");
     const bool recheck = p->recheck != 0 || tc;
-    int rc = ensure_common<F>(ctx, n, d, k, recheck, tc);
-    if (rc) return rc;
-    kmb::UpdatePlan plan = kmb::make_update_plan(n, k, d);
-    if (!kmb::ensure_update_buffers(ctx->ws, plan, sizeof(F))) return fail(ctx, KMB_ENOMEM, "update buffers");
+    const kmb::SmallPlan small = recheck ? kmb::SmallPlan() : kmb::make_small_plan<F>(n, d, k);
+    int rc;
+    kmb::UpdatePlan plan;
+    if (!small.ctas) {
+        if ((rc = ensure_common<F>(ctx, n, d, k, recheck, tc))) return rc;
+        plan = kmb::make_update_plan(n, k, d);
+        if (!kmb::ensure_update_buffers(ctx->ws, plan, sizeof(F))) return fail(ctx, KMB_ENOMEM, "update buffers");
+    }
     kmb::Workspace &ws = ctx->ws;
     cudaStream_t s = ctx->stream;
 
@@ -549,6 +596,29 @@ int train_impl(kmb_context *ctx, int memory, const void *Xv, int64_t n, int64_t 
     if (memory == KMB_MEM_HOST) {
         if ((rc = upload<F>(ctx, ws.X, Xv, sizeof(F) * n * d, &X))) return rc;
         if ((rc = upload<F>(ctx, ws.C0, C0v, sizeof(F) * k * d, &C0))) return rc;
+    }
+    if (small.ctas) {
+        const bool host = memory == KMB_MEM_HOST;
+        if (!ws.ensure(ws.Ccur, sizeof(F) * k * d) || !ws.ensure(ws.labels, sizeof(int32_t) * n))
+            return fail(ctx, KMB_ENOMEM, "device allocation failed (n=%lld d=%lld k=%lld)", (long long)n, (long long)d,
+                        (long long)k);
+        F *C = (host || !C_out) ? (F *)ws.Ccur.ptr : (F *)C_out;
+        int32_t *lab = (host || !responses) ? (int32_t *)ws.labels.ptr : responses;
+        if ((rc = run_small<F>(ctx, small, X, n, d, C0, p, true, C, lab))) return rc;
+        if (host) {
+            if (C_out) KMB_CUDA(cudaMemcpyAsync(C_out, C, sizeof(F) * k * d, cudaMemcpyDeviceToHost, s));
+            if (responses) KMB_CUDA(cudaMemcpyAsync(responses, lab, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, s));
+            KMB_CUDA(cudaStreamSynchronize(s));
+        }
+        const LoopState &hs = ctx->h_state[0];
+        if (objective) *objective = hs.objective;
+        if (iteration_count) *iteration_count = hs.iterations;
+        if (stats) {
+            *stats = kmb_stats();
+            stats->empty_cluster_events = hs.empty_events;
+            stats->last_shift = hs.shift;
+        }
+        return KMB_OK;
     }
     int32_t *labels = (memory == KMB_MEM_DEVICE && responses) ? responses : (int32_t *)ws.labels.ptr;
     F *Ccur = (F *)ws.Ccur.ptr;

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 
 #include "../../include/onedal_b200_kmeans.h"
@@ -39,7 +40,50 @@ struct LoopState {
     int upd_mode;         // 0: recompute from all rows (counting sort), 1: apply the moved rows
     int upd_valid;        // sums, counts and previous labels describe the previous pass
     long long n_moved;    // rows whose label changed in this pass
+    double objective;     // the small train's exact objective (kmb_small.cu)
 };
+
+// Grid-wide barrier of a cooperative launch: count and ticket are zero at its start.
+struct GridSync {
+    unsigned count;   // arrivals since the launch began
+    unsigned ticket;  // CTAs past their last work
+    int error;        // a wait ran out (cleared by the call that owns the state)
+    int pad;
+};
+
+constexpr long long kGridTimeout = 4000000000ll;  // ~2 s of SM clocks per wait
+
+// Every CTA of the grid arrives before any leaves (cooperative launch: all CTAs are
+// resident); `arrived` counts this CTA's barriers, from zero. One release-add and acquire
+// polls of a count that only grows: about 1500 cycles, where a barrier with a generation
+// word, a reset and full fences took 5000. The wait is bounded; false when this CTA's ran
+// out, which is recorded in sy->error (the others' then run out too). Thread 0 decides
+// and the CTA follows, so all its threads take the same path.
+__device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived) {
+    __shared__ int s_grid_ok;
+    __syncthreads();
+    ++arrived;
+    if (gridDim.x == 1) return true;
+    if (threadIdx.x == 0) {
+        const unsigned target = arrived * gridDim.x;
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&sy->count) : "memory");
+        unsigned seen;
+        const long long t0 = clock64();
+        int ok = 1;
+        for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&sy->count) : "memory");
+            if (seen >= target) break;
+            if (clock64() - t0 > kGridTimeout) {
+                atomicExch(&sy->error, 1);
+                ok = 0;
+                break;
+            }
+        }
+        s_grid_ok = ok;
+    }
+    __syncthreads();
+    return s_grid_ok != 0;
+}
 
 // Recheck queue entry written by the assignment kernels for near-tie rows.
 struct RecheckEntry {
@@ -121,6 +165,7 @@ struct Workspace {
     DevBuf sel_state, cand, obj_part, scalars, state;
     DevBuf Xhi, Xlo, Chi, Clo, tcx, rowb, pp_acc, pp_rand, pp_state, pp_flags;
     DevBuf csr_vals, csr_cols64, csr_rowptr64, csr_cols, csr_rowptr, csr_bad, csr_cnorm;
+    DevBuf small;  // kmb_small.cu's scratch
     DevBuf ex_acc, ex_cnt, ex_prev, ex_colexp, ex_records;  // exact update: limb sums, counts, previous
     DevBuf sp_sums, sp_counts, sp_sq, sp_rowsq, sp_Ca, sp_Cb, sp_ids, sp_rows, sp_state, sp_gather;  // kmb_train_spmd
     DevBuf sp_acc, sp_colexp, sp_shift;                                                                // (exact sums)
@@ -251,6 +296,37 @@ template <typename F>
 void launch_update(const F *X, const UpdatePlan &p, const int32_t *labels, const F *d2, F *C_old, F *C_new,
                    Workspace &ws, LoopState *st, bool commit, cudaStream_t s, const CsrRows *csr = nullptr,
                    F *exact_d2 = nullptr);
+
+// ---- small dense problems (plain form): the whole train in one cooperative launch ----
+// Taken when the rows fit the SMs' shared memory, k <= 256, d <= 64 and n * k * d <= 2^30:
+// up to there an iteration's arithmetic is no longer than the 14 launches of the general
+// path (30 us); 100,000 x 20, k = 20 takes 19 us an iteration here and 68 us there.
+constexpr int64_t kSmallTrainMaxK = 256;
+constexpr int64_t kSmallTrainMacs = 1ll << 30;
+struct SmallPlan {
+    int ctas = 0;  // 0: not a small problem
+    int rows = 0;  // per CTA
+};
+template <typename F>
+SmallPlan make_small_plan(int64_t n, int64_t d, int64_t k);
+template <typename F>
+size_t small_scratch_bytes(const SmallPlan &p, int64_t d, int64_t k);
+// What a small train leaves: valid unless sync.error is set.
+struct SmallOut {
+    LoopState st;
+    GridSync sync;
+};
+// C0 (k x d) -> C_out (k x d; may be C0), labels (n, may be null) and the SmallOut at the
+// start of scratch. final_pass: the labels are those under the final centroids and
+// st.objective is set; else they are the last update's. The grid's CTAs wait for one another: launches that do are kept apart by
+// cooperative_mutex until they have ended.
+template <typename F>
+cudaError_t launch_small_train(const SmallPlan &p, const F *X, int64_t n, int64_t d, const F *C0, int64_t k, int64_t T,
+                               double eps, bool final_pass, F *C_out, int32_t *labels, void *scratch, cudaStream_t s);
+// Held by a host thread from a launch that may fill the device with CTAs waiting for one
+// another until that launch has ended, so that two such grids are never partly resident
+// at a time.
+std::mutex &cooperative_mutex();
 
 // ---- exact fixed-point sums (shared by the Lloyd update and the batched form) ----
 // A value x of column t is the integer v = round(x * 2^E_t), |v| < 2^94, E_t =

@@ -374,9 +374,6 @@ template <> struct KeyOf<double> {
     }
 };
 
-// ---- grid-wide barrier of a cooperative launch --------------------------------
-
-constexpr long long kTailTimeout = 4000000000ll;  // ~2 s of SM clocks per barrier wait
 constexpr int kTailThreads = 512;
 constexpr int kTailWarps = kTailThreads / 32;
 constexpr int kSelBits = 11;               // radix-select digit
@@ -384,48 +381,13 @@ constexpr int kSelBins = 1 << kSelBits;
 constexpr int kSelMaxRounds = 6;           // 64-bit keys
 constexpr int kSortSmem = 1024;            // candidates sorted in shared memory up to this many
 
-// Device state of the update's last kernel. count, gen and ticket are left ready for
-// the next launch; the rest is cleared by the launch that uses it.
-struct TailSync {
-    unsigned count;   // barrier arrivals of the current generation
-    unsigned gen;     // barrier generation
-    unsigned ticket;  // CTAs past their last work
-    int error;        // a barrier wait ran out
+// Device state of the update's last kernel. count and ticket are left zero for the next
+// launch; the rest is cleared by the launch that uses it.
+struct TailSync : GridSync {
     unsigned n_cand;  // candidates appended
     unsigned pad[3];
     unsigned hist[kSelMaxRounds][kSelBins];
 };
-
-// Every CTA of the grid arrives before any leaves (cooperative launch: all CTAs are
-// resident). The wait is bounded; false once any CTA gave up. Thread 0 decides and the
-// CTA follows, so all its threads take the same path.
-__device__ __forceinline__ bool tail_sync(TailSync *sy) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile unsigned *vgen = &sy->gen;
-        const unsigned g = *vgen;
-        __threadfence();
-        if (atomicAdd(&sy->count, 1u) == gridDim.x - 1) {
-            sy->count = 0;
-            __threadfence();
-            atomicAdd(&sy->gen, 1u);
-        } else {
-            const long long t0 = clock64();
-            while (*vgen == g) {
-                if (*(volatile int *)&sy->error) break;
-                if (clock64() - t0 > kTailTimeout) {
-                    atomicExch(&sy->error, 1);
-                    break;
-                }
-            }
-        }
-        __threadfence();
-        s_ok = *(volatile int *)&sy->error == 0;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
 
 struct Cand {
     unsigned long long key;
@@ -469,7 +431,8 @@ __device__ void cand_sort(Cand *buf, int P) {
 // 1.8 ms at 10M; with the grid collecting, ten updates that each reseed take 3.5 ms less
 // at 1M x 20, k = 1000 (whole train 11.0 -> 7.5 ms) and 22 ms less at 10M x 64, k = 256.
 template <typename F>
-__device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, Cand *__restrict__ cand) {
+__device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, unsigned &arrived,
+                           Cand *__restrict__ cand) {
     using K = KeyOf<F>;
     __shared__ unsigned s_hist[kSelBins];
     __shared__ unsigned s_scan[kTailWarps];
@@ -503,7 +466,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
         __syncthreads();
         for (int i = tid; i < kSelBins; i += kTailThreads)
             if (s_hist[i]) atomicAdd(&sy->hist[round][i], s_hist[i]);
-        if (!tail_sync(sy)) return false;
+        if (!grid_sync(sy, arrived)) return false;
         // the digit that holds the need-th largest: bins in descending order, four a thread
         unsigned c[4], sum = 0;
 #pragma unroll
@@ -557,7 +520,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
             }
         }
     }
-    if (!tail_sync(sy)) return false;
+    if (!grid_sync(sy, arrived)) return false;
     if (blockIdx.x == 0) {
         if (!all_eq) {
             if (tid == 0) s_base = (unsigned)m - need;
@@ -602,7 +565,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
             cand_sort(cand, P);
         }
     }
-    return tail_sync(sy);
+    return grid_sync(sy, arrived);
 }
 
 // Exact squared distances for the empty-cluster candidates: when some cluster is
@@ -632,7 +595,8 @@ __global__ void refresh_d2_kernel(const F *__restrict__ X, int64_t n, int d, con
 template <typename F>
 __global__ void __launch_bounds__(kTailThreads)
 top_rows_kernel(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, Cand *cand, long long *__restrict__ rows) {
-    if (!select_top<F>(d2, n, m, sy, cand)) return;
+    unsigned arrived = 0;
+    if (!select_top<F>(d2, n, m, sy, arrived, cand)) return;
     if (blockIdx.x == 0)
         for (int e = threadIdx.x; e < m; e += kTailThreads) rows[e] = __ldcg(&cand[e].row);
 }
@@ -708,8 +672,9 @@ __global__ void __launch_bounds__(kTailThreads) update_tail_kernel(const TailArg
                 __syncthreads();
             }
         }
-        ok = tail_sync(a.sy);
-        if (ok) ok = select_top<F>(a.d2, a.n, ne, a.sy, a.cand);
+        unsigned arrived = 0;
+        ok = grid_sync(a.sy, arrived);
+        if (ok) ok = select_top<F>(a.d2, a.n, ne, a.sy, arrived, a.cand);
         if (!ok) {
             if (tid == 0) {
                 st->error = KMB_ETIMEDOUT;
@@ -745,7 +710,7 @@ __global__ void __launch_bounds__(kTailThreads) update_tail_kernel(const TailArg
             }
             __syncthreads();
         }
-        if (a.commit && !tail_sync(a.sy)) {
+        if (a.commit && !grid_sync(a.sy, arrived)) {
             if (tid == 0) {
                 st->error = KMB_ETIMEDOUT;
                 st->done = 1;
@@ -771,6 +736,7 @@ __global__ void __launch_bounds__(kTailThreads) update_tail_kernel(const TailArg
         double tot = 0.0;
         for (int w = 0; w < kTailWarps; ++w) tot += s_red[w];
         a.sy->ticket = 0;
+        a.sy->count = 0;  // (every CTA is past its last barrier)
         st->shift = tot;
         st->empty_events += ne;
         if (a.prev) {  // the maintained sums describe this pass's labels

@@ -1,0 +1,103 @@
+"""Small dense trains in one launch against the general path: the same problem, asked for
+with the FP64 recheck (which the general path alone takes) at values whose near ties are
+exact, so that both give the same responses. Sizes at the edges of the rule and of the
+kernel: one CTA and many, ragged rows per CTA, the padded column counts, one cluster, as
+many clusters as threads allow, fewer rows than clusters would fill, empty clusters over
+several CTAs."""
+import numpy as np
+import pytest
+
+from onedal_b200 import kmeans
+from oracle import restated
+
+pytestmark = pytest.mark.gpu
+
+
+def _data(n, d, k, dt, seed, dup):
+    rng = np.random.default_rng(seed)
+    centres = rng.integers(-40, 41, (k, d))
+    X = (centres[rng.integers(0, k, n)] * 4 + rng.integers(-6, 7, (n, d))).astype(dt)
+    C0 = X[rng.permutation(n)[:k]].copy()
+    if dup and k > 2:
+        C0[k // 2:] = C0[0]  # empty clusters in the first update
+    return X, C0
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k,T,dup", [(1, 1, 1, 3, False), (100, 3, 3, 50, False), (513, 4, 2, 20, False),
+                                         (2047, 24, 7, 20, True), (2049, 33, 40, 10, True), (30_001, 20, 20, 12, False),
+                                         (9_999, 64, 256, 6, True), (148 * 256 + 1, 8, 33, 9, True),
+                                         (60_000, 47, 61, 5, False)])
+def test_equals_the_general_path(dt, n, d, k, T, dup):
+    X, C0 = _data(n, d, k, dt, n + d + k, dup)
+    desc = kmeans.descriptor(dt).set_cluster_count(k).set_max_iteration_count(T)
+    desc.set_compute_form(kmeans.compute_form.plain)
+    a = kmeans.train(desc, X, C0)
+    b = kmeans.train(desc.set_recheck(True), X, C0)
+    assert a.get_iteration_count() == b.get_iteration_count()
+    assert a.stats.empty_cluster_events == b.stats.empty_cluster_events
+    if dt == np.float32:
+        lab, _, _ = restated.assign_f32_in_f64(X, a.get_model().get_centroids())
+        same = (a.get_responses() == b.get_responses()).all()
+        if same:
+            np.testing.assert_array_equal(a.get_model().get_centroids(), b.get_model().get_centroids())
+        assert (a.get_responses().ravel() == lab).mean() > 0.999
+    else:
+        np.testing.assert_array_equal(a.get_responses(), b.get_responses())
+        # sums in another order: n additions of values below M, 2^-53 each, over the count
+        ca, cb = a.get_model().get_centroids(), b.get_model().get_centroids()
+        np.testing.assert_allclose(ca, cb, rtol=0, atol=n * 2.0 ** -52 * np.abs(X).max())
+    fa, fb = a.get_objective_function_value(), b.get_objective_function_value()
+    assert abs(fa - fb) <= 1e-6 * max(fa, fb, 1e-300)
+
+
+def test_empty_clusters_take_the_farthest_rows_over_all_blocks():
+    n, d, k = 148 * 300, 3, 40
+    rng = np.random.default_rng(3)
+    X = rng.integers(-300, 301, (n, d)).astype(np.float64)
+    X[1::2] = X[0::2]  # every distance twice: the lower row first
+    C0 = np.full((k, d), 1e6)
+    C0[0] = 0
+    desc = kmeans.descriptor(np.float64).set_cluster_count(k).set_max_iteration_count(1)
+    r = kmeans.train(desc, X, C0)
+    order = np.lexsort((np.arange(n), -(X ** 2).sum(1)))[:k - 1]
+    np.testing.assert_array_equal(r.get_model().get_centroids()[1:], X[order])
+    assert r.stats.empty_cluster_events == k - 1
+
+
+@pytest.mark.parametrize("span", [1, 40, 80, 120])
+def test_float_sums_are_exact_over_the_exponent_range(span):
+    """Values over 2^span in one column, infinities in another problem: the centroids are the
+    exact integers' (rounded at 2^-94 of the column's largest value), whatever the path."""
+    rng = np.random.default_rng(span)
+    n, d, k = 3000, 5, 4
+    X = (rng.choice([-1.0, 1.0], (n, d)) * 2.0 ** rng.uniform(-span, 0, (n, d))).astype(np.float32)
+    X[0] = 1.0
+    C0 = X[:k].copy()
+    desc = kmeans.descriptor(np.float32).set_cluster_count(k).set_max_iteration_count(1)
+    desc.set_compute_form(kmeans.compute_form.plain)
+    r = kmeans.train(desc, X, C0)
+    lab = kmeans.infer(desc, kmeans.model(C0), X).get_responses().ravel()
+    from fractions import Fraction
+    for j in range(k):
+        rows = X[lab == j]
+        if len(rows) < 2:
+            continue
+        for t in range(d):
+            unit = Fraction(2) ** (int(np.frexp(np.abs(X[:, t]).max())[1]) - 94)
+            total = sum(round(Fraction(float(v)) / unit) for v in rows[:, t]) * unit
+            s = float(total)  # the nearest double
+            want = np.float32(s / len(rows))
+            assert r.get_model().get_centroids()[j, t] == want, (j, t)
+
+
+def test_infinite_rows_take_the_same_sums_as_the_general_path():
+    rng = np.random.default_rng(5)
+    X = rng.standard_normal((2000, 6)).astype(np.float32)
+    X[7, 2] = np.inf
+    X[1500, 0] = np.nan
+    desc = kmeans.descriptor(np.float32).set_cluster_count(5).set_max_iteration_count(2)
+    desc.set_compute_form(kmeans.compute_form.plain)
+    a = kmeans.train(desc, X, X[10:15].copy())
+    b = kmeans.train(desc.set_recheck(True), X, X[10:15].copy())
+    np.testing.assert_array_equal(a.get_model().get_centroids(), b.get_model().get_centroids())
