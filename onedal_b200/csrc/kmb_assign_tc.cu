@@ -1171,6 +1171,10 @@ assign_tc_own_kernel(const __grid_constant__ CUtensorMap tmXh, const __grid_cons
 // best or lie inside the band of the best has y >= that bound - 2e, so the
 // epilogue skips values below thr0 = bound - 2e (rounded down). Without a prior,
 // or for a row without a valid previous label, thr0 = -inf.
+// Computed in FP32, every step rounded away from the exact value on the safe side (up for
+// e, the radius and the band, down for the bound), so rounding only widens the band by a
+// few ulps. Bound by the 20 bytes a row; in FP64 its square roots bounded it (20M rows 284
+// us, 148 us here).
 __global__ void row_bounds_kernel(int64_t n, const float *__restrict__ xnorm, const int32_t *__restrict__ labels,
                                   const float *__restrict__ d2, const double *__restrict__ shift_part,
                                   const double *__restrict__ cnorm_max, const double *__restrict__ cnorm_max_prev,
@@ -1180,56 +1184,99 @@ __global__ void row_bounds_kernel(int64_t n, const float *__restrict__ xnorm, co
     const double u = 5.9604644775390625e-8;  // 2^-24
     const double ub = 3.90625e-3;             // 2^-8
     const double ub2 = 1.52587890625e-5;      // 2^-16
-    const double cmax = *cnorm_max;
-    const double cmax_prev = prior ? *cnorm_max_prev : 0.0;
     // split form: the dropped xl.cl term and the bf16 rounding of the lo parts;
     // single product: |x.c - bf16(x).bf16(c)| <= (2 u_b + u_b^2) sum |x_t c_t|
     const double split = products == 3 ? 3.03 * ub2 : 2.0 * ub + ub2;
     const double acc = split + 2.0 * products * dpad * 2.0 * u;
+    const double cmax = *cnorm_max, cmax_prev = prior ? *cnorm_max_prev : 0.0;
+    // e = ea ||x|| + eb with these coefficients (and ea_p, eb_p under the previous centroids)
+    const float ea = __double2float_ru(1.0625 * (acc + 2.0 * u) * cmax), eb = __double2float_ru(1.0625 * u * cmax * cmax);
+    const float ea_p = __double2float_ru(1.0625 * (acc + 2.0 * u) * cmax_prev);
+    const float eb_p = __double2float_ru(1.0625 * u * cmax_prev * cmax_prev);
+    const float u2 = 1.1920929e-7f;  // 2 u
     for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < n;
          row += (int64_t)gridDim.x * blockDim.x) {
         const float xn = xnorm[row];
-        const double xl = sqrt(fmax((double)xn, 0.0));
-        const double xc = xl * cmax;
-        const double e = 1.0625 * (acc * xc + 2.0 * u * (0.5 * cmax * cmax + xc));
+        const float xl = __fsqrt_ru(fmaxf(xn, 0.0f));
+        const float e = __fmaf_ru(ea, xl, eb);
         float thr0 = __int_as_float(0xff800000);
         const int l = prior ? labels[row] : -1;
         if (l >= 0 && l < k) {
-            const double d2p = (double)d2[row];
-            const double xcp = xl * cmax_prev;
-            const double e_prev = 1.0625 * (acc * xcp + 2.0 * u * (0.5 * cmax_prev * cmax_prev + xcp));
-            const double dsq = fmax(d2p, 0.0) + 2.0 * e_prev + 2.0 * u * (fabs(d2p) + (double)xn);
-            const double rad = sqrt(dsq) + sqrt(shift_part[l]) * (1.0 + 1e-12);
-            const double r2 = rad * rad;
-            const double lb = 0.5 * ((double)xn * (1.0 - 2.0 * u) - r2) - 3.0 * e -
-                              9.5367431640625e-7 * ((double)xn + r2);  // 2^-20 slack for this arithmetic
-            if (lb >= -3.0e38) thr0 = __double2float_rd(lb);          // also rejects NaN
+            const float d2p = d2[row];
+            const float e_prev = __fmaf_ru(ea_p, xl, eb_p);
+            // D_old^2 <= max(d2, 0) + 2 e_prev + 2u (|d2| + ||x||^2)
+            const float dsq = __fadd_ru(fmaxf(d2p, 0.0f), __fmaf_ru(2.0f, e_prev, __fmul_ru(u2, __fadd_ru(fabsf(d2p), xn))));
+            const float moved = __fsqrt_ru(__double2float_ru(shift_part[l] * (1.0 + 1e-12)));
+            const float rad = __fadd_ru(__fsqrt_ru(dsq), moved);
+            const float r2 = __fmul_ru(rad, rad);
+            // 0.5 (||x||^2 (1 - 2u) - r^2) - 3 e, and a slack of 2^-20 as in the bound's derivation
+            const float lo = __fmul_rd(0.5f, __fsub_rd(__fmul_rd(xn, 1.0f - u2), r2));
+            const float lb = __fsub_rd(__fsub_rd(lo, __fmul_ru(3.0f, e)), __fmul_ru(9.5367431640625e-7f, __fadd_ru(xn, r2)));
+            if (lb >= -3.0e38f) thr0 = lb;  // also rejects NaN
         }
-        out[row] = make_float2(thr0, __double2float_ru(2.0 * e));
+        out[row] = make_float2(thr0, __fmul_ru(2.0f, e));
     }
 }
 
-// x -> (bf16(x), bf16(x - bf16(x))) into [rows][dpad] panels, zero padding,
-// and ||x||^2 with the summation order of row_norms_kernel. One warp per row,
-// grid-stride over rows; every element of X is read once.
-__global__ void split_rows_kernel(const float *__restrict__ src, int64_t rows, int d, int dpad,
-                                  __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                                  float *__restrict__ xnorm) {
-    // lo == nullptr: the single-product form reads the hi panels only
-    const int lane = threadIdx.x & 31;
-    const int64_t warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
-        const float *x = src + r * d;
+// x -> (bf16(x), bf16(x - bf16(x))) into [rows][dpad] panels, zero padding, and ||x||^2
+// (FP64 sum of squares rounded to float). Sixteen lanes a row, four columns of every 64 a
+// lane: W floats a load (4: rows of 16-byte multiples at an aligned base, 2: of 8, else 1),
+// 8-byte stores of each panel, every element of X read once; lo == nullptr: hi panels only
+// (the single product). Bound by the HBM bytes; a warp per row with 2-byte stores took 842
+// us for 4M x 128 (4.1 GB) and 534 us for 3M x 50 (1.4 GB): 675 and 297 us here.
+template <int W>
+__global__ void __launch_bounds__(256) split_rows_kernel(const float *__restrict__ src, int64_t rows, int d, int dpad,
+                                                         __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
+                                                         float *__restrict__ xnorm) {
+    const int sub = threadIdx.x & 15;
+    const int64_t groups = ((int64_t)gridDim.x * blockDim.x) >> 4;
+    // the warp's two rows step together (the shuffles below need all lanes)
+    for (int64_t base = (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 2; base < rows; base += groups) {
+        const int64_t r = base + ((threadIdx.x >> 4) & 1);
+        const bool ok = r < rows;
+        const float *x = src + (ok ? r : 0) * d;
+        float v[4][4];
         double s = 0.0;
-        for (int t = lane; t < dpad; t += 32) {
-            const float v = t < d ? x[t] : 0.0f;
-            if (t < d) s += (double)v * (double)v;
-            const __nv_bfloat16 h = __float2bfloat16_rn(v);
-            hi[r * dpad + t] = h;
-            if (lo) lo[r * dpad + t] = __float2bfloat16_rn(v - __bfloat162float(h));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {  // up to 256 columns, all loads before the first use
+            const int t = 64 * q + 4 * sub;
+#pragma unroll
+            for (int i = 0; i < 4; i += W) {
+                const bool in = ok && t + i < d;  // (W divides d)
+                if constexpr (W == 4) {
+                    const float4 f = in ? __ldcs(reinterpret_cast<const float4 *>(x + t)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    v[q][0] = f.x, v[q][1] = f.y, v[q][2] = f.z, v[q][3] = f.w;
+                } else if constexpr (W == 2) {
+                    const float2 f = in ? __ldcs(reinterpret_cast<const float2 *>(x + t + i)) : make_float2(0.f, 0.f);
+                    v[q][i] = f.x, v[q][i + 1] = f.y;
+                } else {
+                    v[q][i] = in ? __ldcs(x + t + i) : 0.0f;
+                }
+            }
         }
-        for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
-        if (lane == 0) xnorm[r] = (float)s;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int t = 64 * q + 4 * sub;
+            if (!ok || t >= dpad) continue;
+            __nv_bfloat162 h2[2], l2[2];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                s = fma((double)v[q][i], (double)v[q][i], s);
+                const __nv_bfloat16 h = __float2bfloat16_rn(v[q][i]);
+                const __nv_bfloat16 l = __float2bfloat16_rn(v[q][i] - __bfloat162float(h));
+                if (i & 1) {
+                    h2[i >> 1].y = h;
+                    l2[i >> 1].y = l;
+                } else {
+                    h2[i >> 1].x = h;
+                    l2[i >> 1].x = l;
+                }
+            }
+            *reinterpret_cast<uint2 *>(hi + r * dpad + t) = *reinterpret_cast<const uint2 *>(h2);
+            if (lo) *reinterpret_cast<uint2 *>(lo + r * dpad + t) = *reinterpret_cast<const uint2 *>(l2);
+        }
+        for (int m = 8; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+        if (ok && sub == 0) xnorm[r] = (float)s;
     }
 }
 
@@ -1287,9 +1334,10 @@ void launch_split_rows(const float *X, int64_t rows, int64_t d, void *hi, void *
                        cudaStream_t s) {
     if (rows == 0) return;
     const int64_t dpad = tc_dpad(d);
-    const int blocks = (int)std::min<int64_t>((rows * 32 + 255) / 256, (int64_t)num_sms * 16);
-    tc::split_rows_kernel<<<blocks, 256, 0, s>>>(X, rows, (int)d, (int)dpad, (__nv_bfloat16 *)hi, (__nv_bfloat16 *)lo,
-                                                 xnorm);
+    const int blocks = (int)std::min<int64_t>((rows * 16 + 255) / 256, (int64_t)num_sms * 16);
+    const int w = d % 4 == 0 && (uintptr_t)X % 16 == 0 ? 4 : d % 2 == 0 && (uintptr_t)X % 8 == 0 ? 2 : 1;
+    auto kern = w == 4 ? tc::split_rows_kernel<4> : w == 2 ? tc::split_rows_kernel<2> : tc::split_rows_kernel<1>;
+    kern<<<blocks, 256, 0, s>>>(X, rows, (int)d, (int)dpad, (__nv_bfloat16 *)hi, (__nv_bfloat16 *)lo, xnorm);
     KMB_LAUNCHED();
 }
 

@@ -386,6 +386,99 @@ __global__ void __launch_bounds__(kUpdWarps * 32)
     }
 }
 
+// The distance update for the rows that neither of the above reads well: lengths that are
+// no 16-byte multiple, or shorter than a segment, at a 16-byte aligned base. A group's 32
+// rows are one contiguous range (32 * row bytes, a multiple of 16), so it goes global ->
+// shared in 16-byte pieces at the rows' own pitch, fully coalesced, in a ring of kRowStages
+// groups per warp; each lane then folds its row in coordinate order, W values a read. Bound
+// by the row bytes: 3M x 50, 180 us by 128-byte segments through registers, 150 us here.
+constexpr int kRowStages = 3;
+constexpr int kRowsMaxSmem = 112 * 1024;  // two CTAs per SM: d <= 69 (float)
+
+template <typename F>
+__host__ __device__ constexpr int rows_warp_smem(int d) {
+    return kRowStages * 32 * d * (int)sizeof(F) + kPPBlock * (int)sizeof(F);
+}
+
+template <typename F, int W>
+__global__ void __launch_bounds__(kUpdWarps * 32)
+    pp_update_rows_kernel(const F *__restrict__ X, int64_t n, int d, int64_t nb, const F *__restrict__ center,
+                          F *__restrict__ md, F *__restrict__ acc, unsigned *__restrict__ flags, unsigned epoch,
+                          PPState *st) {
+    extern __shared__ __align__(16) unsigned char pp_rows_smem[];
+    if (st->stopped) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (blockIdx.x == 0) {  // the leading CTA folds the overall sum
+        if (warp == 0) fold_overall(acc, flags, nb, epoch, st);
+        return;
+    }
+    F *cs = (F *)pp_rows_smem;  // the center, padded to 16 bytes
+    const int cpad = (d * (int)sizeof(F) + 15) / 16 * 16;
+    for (int i = threadIdx.x; i < d; i += kUpdWarps * 32) cs[i] = center[i];
+    __syncthreads();
+    const int64_t b = (int64_t)(blockIdx.x - 1) * kUpdWarps + warp;
+    if (b >= nb) return;  // warp-uniform; no CTA-wide barrier below
+    unsigned char *ws = pp_rows_smem + cpad + (size_t)warp * rows_warp_smem<F>(d);
+    const int gbytes = 32 * d * (int)sizeof(F);
+    F *s_md = (F *)(ws + kRowStages * gbytes);
+    const int64_t base = b * kPPBlock;
+    const int cnt = (int)min((int64_t)kPPBlock, n - base);
+    const int ngroups = (cnt + 31) / 32;
+    auto issue = [&](int g) {
+        if (g < ngroups) {
+            const unsigned char *src = (const unsigned char *)(X + (base + (int64_t)g * 32) * d);
+            unsigned char *dst = ws + (g % kRowStages) * gbytes;
+            const int bytes = min(32, cnt - g * 32) * d * (int)sizeof(F);  // (no read past the last row)
+            for (int o = lane * 16; o < bytes; o += 512)
+                cp_async16(dst + o, src + o, min(16, bytes - o));
+        }
+        cp_async_commit();
+    };
+    for (int g = 0; g < kRowStages - 1; ++g) issue(g);
+    struct alignas(sizeof(F) * W) Vec { F v[W]; };
+    for (int g = 0; g < ngroups; ++g) {
+        issue(g + kRowStages - 1);
+        const int r = g * 32 + lane;
+        const F old = r < cnt ? md[base + r] : F(0);
+        cp_async_wait<kRowStages - 1>();
+        __syncwarp();
+        const F *x = (const F *)(ws + (g % kRowStages) * gbytes) + lane * d;
+        F d2 = F(0);
+#pragma unroll 4
+        for (int i = 0; i < d; i += W) {
+            const Vec xv = *reinterpret_cast<const Vec *>(x + i), cv = *reinterpret_cast<const Vec *>(cs + i);
+#pragma unroll
+            for (int u = 0; u < W; ++u) {
+                const F e = xv.v[u] - cv.v[u];
+                d2 = fma(e, e, d2);
+            }
+        }
+        if (r < cnt) {
+            const F m = !(d2 < old) ? old : d2;  // the reference's min(best, d2)
+            md[base + r] = m;
+            s_md[r] = m;
+        }
+        __syncwarp();
+    }
+    cp_async_wait<0>();
+    __syncwarp();
+    if (lane == 0) {
+        constexpr int V = 16 / (int)sizeof(F);
+        using V16 = typename std::conditional<sizeof(F) == 4, float4, double2>::type;
+        F sum = F(0);
+        int i = 0;
+#pragma unroll 4
+        for (; i + V <= cnt; i += V) {
+            const V16 q = *reinterpret_cast<const V16 *>(s_md + i);
+            const F *e = reinterpret_cast<const F *>(&q);
+#pragma unroll
+            for (int u = 0; u < V; ++u) sum += e[u];
+        }
+        for (; i < cnt; ++i) sum += s_md[i];
+        publish_block_sum(acc, flags, b, sum, epoch);
+    }
+}
+
 constexpr int kSelThreads = 256;
 
 // Eight consecutive values from 16-byte aligned shared memory in 16-byte loads.
@@ -640,9 +733,18 @@ void launch_pp_rounds(const F *X, int64_t n, int64_t d, int64_t k, int64_t c_beg
                        d >= 128 / (int64_t)sizeof(F);
     const int async_smem = kUpdWarps * async_warp_smem<F>();
     if (async) cudaFuncSetAttribute(pp_update_async_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, async_smem);
+    // other rows at a 16-byte aligned base whose groups fit shared memory: contiguous groups
+    const int rows_smem = (int)((d * sizeof(F) + 15) / 16 * 16) + kUpdWarps * rows_warp_smem<F>((int)std::min<int64_t>(d, 1 << 12));
+    const int w = (d * sizeof(F)) % 16 == 0 ? 16 / (int)sizeof(F) : d % 2 == 0 && sizeof(F) == 4 ? 2 : 1;
+    auto rows_kernel = w == 1 ? pp_update_rows_kernel<F, 1> : w == 2 ? pp_update_rows_kernel<F, 2> : pp_update_rows_kernel<F, 16 / (int)sizeof(F)>;
+    const bool rows = !async && ((uintptr_t)X % 16) == 0 && d <= (1 << 12) && rows_smem <= kRowsMaxSmem &&
+                      cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem) == cudaSuccess;
     for (int64_t c = c_begin; c < k; ++c) {
         if (c > c_begin || update_first) {
-            if (async)
+            if (rows)
+                rows_kernel<<<grid, kUpdWarps * 32, rows_smem, s>>>(X, n, (int)d, nb, C + (c - 1) * d, md, acc, flags,
+                                                                    (unsigned)c, st);
+            else if (async)
                 pp_update_async_kernel<F><<<grid, kUpdWarps * 32, async_smem, s>>>(
                     X, n, (int)d, nb, C + (c - 1) * d, md, acc, flags, (unsigned)c, st);
             else

@@ -217,8 +217,8 @@ cudaError_t pool_alloc(void **p, size_t bytes, int dev, cudaStream_t s);
 int tc_tile_n(int64_t k);      // cluster tile of the tensor-core kernel: 128 or 256
 int64_t tc_kpad(int64_t k);   // k rounded up to a multiple of tc_tile_n(k)
 bool tc_supported(int64_t d); // dpad <= 256
-// x -> BF16 hi/lo panels [rows][dpad] (lo may be null: hi only) and ||x||^2 (the
-// same value launch_row_norms gives).
+// x -> BF16 hi/lo panels [rows][dpad] (lo may be null: hi only; dpad <= 256) and ||x||^2
+// (an FP64 sum rounded to float, as launch_row_norms's but in another order).
 void launch_split_rows(const float *X, int64_t rows, int64_t d, void *hi, void *lo, float *xnorm, int num_sms,
                        cudaStream_t s);
 // C -> Chi/Clo [kpad][dpad], -h = -0.5||c||^2 (kpad, -inf padding), max ||c|| (the
@@ -383,6 +383,53 @@ __device__ __forceinline__ Limbs fixed_of(float x, int e) {
     L.l2 = l2;
     return L;
 }
+
+// The exact sum of a column's finite floats in three FP64 bins: the integers of fixed_of,
+// which costs several times the instructions a value. For columns with a finite largest
+// value and e = 94 - ex != 0. With every |x| < 2^ex, a value is
+// hi + mid + low: hi its nearest multiple of 2^(ex - 35), mid the rest's nearest multiple
+// of 2^(ex - 71), low the rest rounded to a multiple of 2^(ex - 94), half to even -- the
+// rounding of fixed_of, whose integer is hi + mid + low in units of 2^(ex - 94) = 2^-e.
+// Adding and subtracting 1.5 * 2^(52 + a) rounds to multiples of 2^a; the remainders are
+// exact, and fewer than 2^16 addends keep each bin's sum below 2^53 of its units.
+struct Bins {
+    double hi = 0.0, mid = 0.0, low = 0.0;
+    struct Magic {
+        double a, b, c;
+        __device__ __forceinline__ explicit Magic(int e)
+            : a(ldexp(1.5, 52 + 59 - e)), b(ldexp(1.5, 52 + 23 - e)), c(ldexp(1.5, 52 - e)) {}
+    };
+    __device__ __forceinline__ void add(float x, const Magic &m3) {
+        const double v = (double)x;
+        const double h = __dadd_rn(__dadd_rn(v, m3.a), -m3.a);
+        hi += h;
+        const double r = v - h;
+        if (r == 0.0) return;  // (nearly always: 24 significant bits)
+        const double m = __dadd_rn(__dadd_rn(r, m3.b), -m3.b);
+        mid += m;
+        const double q = r - m;
+        if (q != 0.0) low += __dadd_rn(__dadd_rn(q, m3.c), -m3.c);
+    }
+    // v * 2^e, an integer below 2^126
+    static __device__ __forceinline__ __int128 scaled(double v, int e) {
+        if (v == 0.0) return 0;
+        const long long bits = __double_as_longlong(v);
+        const int sh = (int)((bits >> 52) & 0x7ff) - 1075 + e;  // (v is normal: a multiple of 2^-243)
+        const unsigned long long m = ((unsigned long long)bits & 0xfffffffffffffull) | 0x10000000000000ull;
+        const __int128 a = sh >= 0 ? (__int128)((unsigned __int128)m << sh) : (__int128)(m >> -sh);
+        return bits < 0 ? -a : a;
+    }
+    // (a non-finite addend leaves hi + mid + low non-finite)
+    __device__ __forceinline__ bool finite() const { return isfinite(hi + mid + low); }
+    __device__ __forceinline__ Limbs limbs(int e) const {
+        const __int128 S = scaled(hi, e) + scaled(mid, e) + scaled(low, e);
+        Limbs l;
+        l.l0 = (long long)(S & 0xffffffffll);
+        l.l1 = (long long)((S >> 32) & 0xffffffffll);
+        l.l2 = (long long)(S >> 64);
+        return l;
+    }
+};
 
 // The nearest double to |m| (round half to even), m < 2^127.
 __device__ __forceinline__ double u128_to_double(unsigned __int128 m) {

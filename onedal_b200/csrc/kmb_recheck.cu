@@ -19,9 +19,9 @@ namespace {
 // of ||c||^2 and x.c for both candidates in double (consecutive lanes read
 // consecutive floats of the row and of each centroid), then three butterfly
 // steps give the group's totals; both candidates' sums have the same
-// association, so equal centroids give equal scores. With VEC (float rows, d a
-// multiple of 4, 16-byte aligned bases) lane l reads 16 bytes at a time
-// (t = 4l .. 4l+3, then 32 further), a quarter of the loads in flight per row.
+// association, so equal centroids give equal scores. With W = 4 or 2 (float rows, d a
+// multiple of W, 4 W-byte aligned bases) lane l reads W values at a time, a W-th of the
+// loads per row.
 template <typename F>
 __device__ __forceinline__ void pair_sums(const F *x, const F *ca, const F *cb, int d, int sub, double &cca,
                                           double &xca, double &ccb, double &xcb) {
@@ -33,8 +33,14 @@ __device__ __forceinline__ void pair_sums(const F *x, const F *ca, const F *cb, 
         xcb = fma(xv, vb, xcb);
     }
 }
+// (the values of a load are converted together before the sums: the same loop with the
+// conversions inside the sums ran five times slower)
+template <int W>
 __device__ __forceinline__ void pair_sums_vec(const float *x, const float *ca, const float *cb, int d, int sub,
-                                              double &cca, double &xca, double &ccb, double &xcb) {
+                                              double &cca, double &xca, double &ccb, double &xcb);
+template <>
+__device__ __forceinline__ void pair_sums_vec<4>(const float *x, const float *ca, const float *cb, int d, int sub,
+                                                 double &cca, double &xca, double &ccb, double &xcb) {
     const float4 *x4 = reinterpret_cast<const float4 *>(x), *a4 = reinterpret_cast<const float4 *>(ca),
                  *b4 = reinterpret_cast<const float4 *>(cb);
 #pragma unroll 4
@@ -51,8 +57,26 @@ __device__ __forceinline__ void pair_sums_vec(const float *x, const float *ca, c
         }
     }
 }
+template <>
+__device__ __forceinline__ void pair_sums_vec<2>(const float *x, const float *ca, const float *cb, int d, int sub,
+                                                 double &cca, double &xca, double &ccb, double &xcb) {
+    const float2 *x2 = reinterpret_cast<const float2 *>(x), *a2 = reinterpret_cast<const float2 *>(ca),
+                 *b2 = reinterpret_cast<const float2 *>(cb);
+#pragma unroll 4
+    for (int t = sub; t < (d >> 1); t += 8) {
+        const float2 xq = x2[t], aq = a2[t], bq = b2[t];
+        const double xv[2] = {xq.x, xq.y}, va[2] = {aq.x, aq.y}, vb[2] = {bq.x, bq.y};
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            cca = fma(va[i], va[i], cca);
+            xca = fma(xv[i], va[i], xca);
+            ccb = fma(vb[i], vb[i], ccb);
+            xcb = fma(xv[i], vb[i], xcb);
+        }
+    }
+}
 
-template <typename F, bool VEC>
+template <typename F, int W>
 __global__ void __launch_bounds__(256) recheck_pairs_kernel(const F *__restrict__ X, int d, const F *__restrict__ C,
                                                             const RecheckEntry *__restrict__ queue,
                                                             int32_t *__restrict__ labels, F *__restrict__ d2,
@@ -78,8 +102,8 @@ __global__ void __launch_bounds__(256) recheck_pairs_kernel(const F *__restrict_
             const F *x = X + (int64_t)q.row * d;
             const F *ca = C + (int64_t)a * d;
             const F *cb = C + (int64_t)b * d;
-            if constexpr (VEC)
-                pair_sums_vec(x, ca, cb, d, sub, cca, xca, ccb, xcb);
+            if constexpr (W > 1)
+                pair_sums_vec<W>(x, ca, cb, d, sub, cca, xca, ccb, xcb);
             else
                 pair_sums(x, ca, cb, d, sub, cca, xca, ccb, xcb);
         }
@@ -324,15 +348,14 @@ constexpr int kFullRows = 8;
 template <typename F>
 void launch_recheck(const F *X, int64_t n, int64_t d, const F *C, int64_t k, const RecheckEntry *queue,
                     int32_t *labels, F *d2, const F *xnorm, LoopState *st, int num_sms, cudaStream_t s) {
-    bool vec = false;
     const bool vec_c = sizeof(F) == 4 && d % 4 == 0 && (uintptr_t)C % 16 == 0;
+    const uintptr_t both = (uintptr_t)X | (uintptr_t)C;
+    const int w = sizeof(F) != 4 ? 1 : d % 4 == 0 && both % 16 == 0 ? 4 : d % 2 == 0 && both % 8 == 0 ? 2 : 1;
     if constexpr (sizeof(F) == 4) {
-        vec = d % 4 == 0 && (uintptr_t)X % 16 == 0 && (uintptr_t)C % 16 == 0;
-        if (vec)
-            recheck_pairs_kernel<float, true><<<num_sms * 8, 256, 0, s>>>(X, (int)d, C, queue, labels, d2, xnorm, st);
+        if (w == 4) recheck_pairs_kernel<F, 4><<<num_sms * 8, 256, 0, s>>>(X, (int)d, C, queue, labels, d2, xnorm, st);
+        if (w == 2) recheck_pairs_kernel<F, 2><<<num_sms * 8, 256, 0, s>>>(X, (int)d, C, queue, labels, d2, xnorm, st);
     }
-    if (!vec)
-        recheck_pairs_kernel<F, false><<<num_sms * 8, 256, 0, s>>>(X, (int)d, C, queue, labels, d2, xnorm, st);
+    if (w == 1) recheck_pairs_kernel<F, 1><<<num_sms * 8, 256, 0, s>>>(X, (int)d, C, queue, labels, d2, xnorm, st);
     KMB_LAUNCHED();
     const size_t rows_smem = (size_t)kFullRows * d * sizeof(F);
     if (rows_smem <= 48 * 1024) {

@@ -306,41 +306,6 @@ __device__ __forceinline__ void acc_add(Acc<float> &a, float x, int e) {
 }
 __device__ __forceinline__ void acc_add(Acc<double> &a, double x, int) { a.v[0] += x; }
 
-// The exact sum of a column's finite floats in three FP64 bins (fixed_of costs some 100
-// instructions a value and bounded the accumulation). With every |x| < 2^ex, a value is
-// hi + mid + low: hi its nearest multiple of 2^(ex - 35), mid the rest's nearest multiple
-// of 2^(ex - 71), low the rest rounded to a multiple of 2^(ex - 94), half to even -- the
-// rounding of fixed_of, whose integer is hi + mid + low in units of 2^(ex - 94) = 2^-e.
-// Adding and subtracting 1.5 * 2^(52 + a) rounds to multiples of 2^a; the remainders are
-// exact, and fewer than 2^16 addends keep each bin's sum below 2^53 of its units.
-struct Bins {
-    double hi = 0.0, mid = 0.0, low = 0.0;
-    __device__ __forceinline__ void add(float x, double ma, double mb, double mc) {
-        const double v = (double)x;
-        const double h = __dadd_rn(__dadd_rn(v, ma), -ma);
-        hi += h;
-        const double r = v - h;
-        if (r == 0.0) return;  // (nearly always: 24 significant bits)
-        const double m = __dadd_rn(__dadd_rn(r, mb), -mb);
-        mid += m;
-        const double q = r - m;
-        if (q != 0.0) low += __dadd_rn(__dadd_rn(q, mc), -mc);
-    }
-    // v * 2^e, an integer below 2^126
-    static __device__ __forceinline__ __int128 scaled(double v, int e) {
-        if (v == 0.0) return 0;
-        const long long bits = __double_as_longlong(v);
-        const int sh = (int)((bits >> 52) & 0x7ff) - 1075 + e;  // (v is normal: a multiple of 2^-243)
-        const unsigned long long m = ((unsigned long long)bits & 0xfffffffffffffull) | 0x10000000000000ull;
-        const __int128 a = sh >= 0 ? (__int128)((unsigned __int128)m << sh) : (__int128)(m >> -sh);
-        return bits < 0 ? -a : a;
-    }
-    __device__ __forceinline__ Acc<float> limbs(int e) const {
-        const __int128 S = scaled(hi, e) + scaled(mid, e) + scaled(low, e);
-        return Acc<float>{{(long long)(S & 0xffffffffll), (long long)((S >> 32) & 0xffffffffll), (long long)(S >> 64)}};
-    }
-};
-
 // The centroid value of summed parts.
 __device__ __forceinline__ float centroid_of(const Acc<float> &a, int e, int count) {
     const __int128 S = ((__int128)a.v[2] << 64) + ((__int128)a.v[1] << 32) + (__int128)a.v[0];
@@ -379,7 +344,7 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
         Xs[r * ds + t] = x;
         infinite |= !isfinite(x);
     }
-    // (the bins take finite values; a CTA with others converts every value by fixed_of)
+    // (the bins take finite values of a finite column, e != 0; fixed_of takes the others)
     const bool finite = __syncthreads_or(infinite) == 0;
     for (int i = tid; i < k4 * DMAX; i += kNT) {
         const int j = i / DMAX, t = i % DMAX;
@@ -446,18 +411,19 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
             Acc<F> v = {};
             const int e = sizeof(F) == 4 ? s_exp[t] : 0;
             if constexpr (sizeof(F) == 4) {
-                if (finite) {
-                    const double ma = ldexp(1.5, 52 + 59 - e), mb = ldexp(1.5, 52 + 23 - e), mc = ldexp(1.5, 52 - e);
+                if (finite && e != 0) {
+                    const Bins::Magic mg(e);
                     Bins bins;
                     for (; i + 4 <= hi; i += 4) {
                         F x[4];
 #pragma unroll
                         for (int q = 0; q < 4; ++q) x[q] = Xs[order[i + q] * ds + t];
 #pragma unroll
-                        for (int q = 0; q < 4; ++q) bins.add(x[q], ma, mb, mc);
+                        for (int q = 0; q < 4; ++q) bins.add(x[q], mg);
                     }
-                    for (; i < hi; ++i) bins.add(Xs[order[i] * ds + t], ma, mb, mc);
-                    return bins.limbs(e);
+                    for (; i < hi; ++i) bins.add(Xs[order[i] * ds + t], mg);
+                    const Limbs l = bins.limbs(e);
+                    return Acc<float>{{l.l0, l.l1, l.l2}};
                 }
             }
             for (; i + 4 <= hi; i += 4) {

@@ -21,6 +21,7 @@
 #include "kmb_internal.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace kmb {
 namespace {
@@ -303,7 +304,8 @@ __device__ __forceinline__ double piece_sum(const double *__restrict__ records, 
     return S;
 }
 
-constexpr int kFinalizeCols = 128;  // columns per finalize block (one per thread)
+constexpr int kFinalizeCols = 128;  // columns per finalize block
+constexpr int kFinalizeThreads = 512;  // of the exact finalize: four or more per column
 
 // Block (j, tile): S = sum of cluster j's pieces (in order) for the tile's
 // columns; c = F(S / count); the tile's shift part. One large cluster thus
@@ -752,40 +754,61 @@ __global__ void __launch_bounds__(kTailThreads) update_tail_kernel(const TailArg
 
 // ---- objective -------------------------------------------------------------
 
-template <typename F>
+// Block b sums its contiguous range of rows: L lanes a row, W values a load; FP64, fixed
+// order. Bound by the row bytes and the float conversions; a thread per column and row took
+// 788 us for 4M x 128 (2.05 GB), 295 us for 3M x 50, 61 us for 1M x 20 and 999 us for 10M x
+// 64: 460, 208, 34 and 553 us here (two or four rows in flight per lane group were slower).
+template <typename F, int W, int L>
 __global__ void __launch_bounds__(256)
 objective_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restrict__ C, const int32_t *__restrict__ labels,
                  double *__restrict__ partials) {
-    constexpr int NT = 256;
-    __shared__ double part[NT];
-    int dl, rp;
-    row_layout(d, NT, dl, rp);
-    const int t = threadIdx.x % dl, rr = threadIdx.x / dl;
+    constexpr int RP = 32 / L;  // rows a warp reads side by side
+    __shared__ double part[8];
+    struct alignas(sizeof(F) * W) Vec { F v[W]; };
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % L, group = lane / L;
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t b = (int64_t)blockIdx.x * per, e = min(n, b + per);
     double acc = 0.0;
-    for (int t0 = 0; t0 < d; t0 += dl) {
-        const int col = t0 + t;
-        if (col >= d) continue;
-        for (int64_t i = b + rr; i < e; i += rp) {
-            const double df = (double)X[i * d + col] - (double)C[(int64_t)labels[i] * d + col];
-            acc += df * df;
+    for (int64_t r = b + (int64_t)warp * RP + group; r < e; r += 8 * RP) {
+        const F *x = X + r * d, *c = C + (int64_t)labels[r] * d;
+        for (int t = sub * W; t < d; t += L * W) {
+            const Vec xv = *reinterpret_cast<const Vec *>(x + t), cv = *reinterpret_cast<const Vec *>(c + t);
+            double xd[W], cd[W];
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                xd[i] = (double)xv.v[i];
+                cd[i] = (double)cv.v[i];
+            }
+#pragma unroll
+            for (int i = 0; i < W; ++i) {
+                const double df = xd[i] - cd[i];
+                acc = fma(df, df, acc);
+            }
         }
     }
-    part[threadIdx.x] = acc;
+    for (int m = 16; m >= 1; m >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, m);
+    if (lane == 0) part[warp] = acc;
     __syncthreads();
-    for (int s = NT / 2; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) part[threadIdx.x] += part[threadIdx.x + s];
-        __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int w = 0; w < 8; ++w) s += part[w];
+        partials[blockIdx.x] = s;
     }
-    if (threadIdx.x == 0) partials[blockIdx.x] = part[0];
 }
 
-__global__ void sum_partials_kernel(const double *__restrict__ partials, int count, double *__restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int i = 0; i < count; ++i) s += partials[i];
-        *out = s;
+// One block, a fixed order.
+__global__ void __launch_bounds__(256) sum_partials_kernel(const double *__restrict__ partials, int count,
+                                                           double *__restrict__ out) {
+    __shared__ double part[8];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < count; i += 256) s += partials[i];
+    for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += part[w];
+        *out = t;
     }
 }
 
@@ -980,9 +1003,20 @@ __global__ void count_moved_kernel(const int32_t *__restrict__ labels, const int
     if (threadIdx.x == 0) s_cnt = 0;
     __syncthreads();
     int c = 0;
-    if (st->upd_valid)
-        for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x)
-            c += labels[r] != prev[r];
+    if (st->upd_valid) {
+        const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+        for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += 8 * stride) {
+            int l[8], p[8];  // sixteen loads in flight
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                const bool in = r + q * stride < n;
+                l[q] = in ? labels[r + q * stride] : 0;
+                p[q] = in ? prev[r + q * stride] : 0;
+            }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) c += l[q] != p[q];
+        }
+    }
     c = __reduce_add_sync(0xffffffffu, c);
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(&s_cnt, c);
     __syncthreads();
@@ -1001,7 +1035,9 @@ __global__ void count_moved_kernel(const int32_t *__restrict__ labels, const int
 }
 
 // Block p sums piece p's rows (one cluster's rows in row order) as integers.
-// records: three limb planes of (pieces x d) int64.
+// records: three limb planes of (pieces x d) int64. Bound by the gathered row reads;
+// converting every value to limbs bounded it (20M x 128: 2.7 ms a full pass, 1.15 ms
+// with the bins).
 __global__ void __launch_bounds__(128)
 segsum_fixed_kernel(const float *__restrict__ X, int d, int k, const int32_t *__restrict__ perm,
                     const int64_t *__restrict__ offsets, const int64_t *__restrict__ piece_base, int64_t piece_rows,
@@ -1031,32 +1067,36 @@ segsum_fixed_kernel(const float *__restrict__ X, int d, int k, const int32_t *__
     const int64_t plane = max_pieces * (int64_t)d;
     for (int t0 = 0; t0 < d; t0 += dl) {
         const int col = t0 + t;
-        long long a0 = 0, a1 = 0, a2 = 0;
+        Limbs a = {0, 0, 0};
         if (col < d) {
             const int ex = colexp[col];
-            int i = rr;
-            for (; i + 7 * rp < cnt; i += 8 * rp) {  // eight gathered loads in flight per thread
-                float v[8];
+            Bins bins;
+            if (ex != 0) {
+                const Bins::Magic mg(ex);
+                int i = rr;
+                for (; i + 7 * rp < cnt; i += 8 * rp) {  // eight gathered loads in flight per thread
+                    float v[8];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) v[u] = X[(int64_t)rows[i + u * rp] * d + col];
+                    for (int u = 0; u < 8; ++u) v[u] = X[(int64_t)rows[i + u * rp] * d + col];
 #pragma unroll
-                for (int u = 0; u < 8; ++u) {
-                    const Limbs L = fixed_of(v[u], ex);
-                    a0 += L.l0;
-                    a1 += L.l1;
-                    a2 += L.l2;
+                    for (int u = 0; u < 8; ++u) bins.add(v[u], mg);
+                }
+                for (; i < cnt; i += rp) bins.add(X[(int64_t)rows[i] * d + col], mg);
+            }
+            if (ex != 0 && bins.finite()) {
+                a = bins.limbs(ex);
+            } else {  // a column of zeros, or non-finite values
+                for (int i = rr; i < cnt; i += rp) {
+                    const Limbs L = fixed_of(X[(int64_t)rows[i] * d + col], ex);
+                    a.l0 += L.l0;
+                    a.l1 += L.l1;
+                    a.l2 += L.l2;
                 }
             }
-            for (; i < cnt; i += rp) {
-                const Limbs L = fixed_of(X[(int64_t)rows[i] * d + col], ex);
-                a0 += L.l0;
-                a1 += L.l1;
-                a2 += L.l2;
-            }
         }
-        part[0][threadIdx.x] = a0;
-        part[1][threadIdx.x] = a1;
-        part[2][threadIdx.x] = a2;
+        part[0][threadIdx.x] = a.l0;
+        part[1][threadIdx.x] = a.l1;
+        part[2][threadIdx.x] = a.l2;
         __syncthreads();
         if (rr == 0 && col < d) {
             long long t0s = part[0][t], t1s = part[1][t], t2s = part[2][t];
@@ -1101,12 +1141,19 @@ __global__ void apply_moves_kernel(const float *__restrict__ X, int64_t n, int d
             for (int t = lane; t < d; t += 32) {
                 const Limbs L = fixed_of(x[t], colexp[t]);
                 const int64_t in = (int64_t)nl * d + t, out = (int64_t)ol * d + t;
-                atomicAdd(&acc[in], (unsigned long long)L.l0);
-                atomicAdd(&acc[plane + in], (unsigned long long)L.l1);
-                atomicAdd(&acc[2 * plane + in], (unsigned long long)L.l2);
-                atomicAdd(&acc[out], (unsigned long long)-L.l0);
-                atomicAdd(&acc[plane + out], (unsigned long long)-L.l1);
-                atomicAdd(&acc[2 * plane + out], (unsigned long long)-L.l2);
+                // (a float's 24 bits span at most two limbs: a third of the atomics is left out)
+                if (L.l0) {
+                    atomicAdd(&acc[in], (unsigned long long)L.l0);
+                    atomicAdd(&acc[out], (unsigned long long)-L.l0);
+                }
+                if (L.l1) {
+                    atomicAdd(&acc[plane + in], (unsigned long long)L.l1);
+                    atomicAdd(&acc[plane + out], (unsigned long long)-L.l1);
+                }
+                if (L.l2) {
+                    atomicAdd(&acc[2 * plane + in], (unsigned long long)L.l2);
+                    atomicAdd(&acc[2 * plane + out], (unsigned long long)-L.l2);
+                }
             }
             if (lane == 0) {
                 atomicAdd(&cnt[nl], 1ull);
@@ -1121,31 +1168,49 @@ __global__ void apply_moves_kernel(const float *__restrict__ X, int64_t n, int d
 // from_acc:
 // the maintained ones), normalised and kept; c = F(S * 2^-E / count) in FP64; the
 // tile's shift part and the empty flag, as finalize_kernel.
-__global__ void __launch_bounds__(kFinalizeCols)
+__global__ void __launch_bounds__(kFinalizeThreads)
 finalize_exact_kernel(const long long *__restrict__ records, int64_t max_pieces, const int64_t *__restrict__ counts_sort,
                       const int64_t *__restrict__ piece_base, const int *__restrict__ colexp, int k,
                       long long *__restrict__ lacc, long long *__restrict__ cnt, const float *__restrict__ C_old,
                       float *__restrict__ C_new, int d, double *__restrict__ shift_tiles,
                       int32_t *__restrict__ empty_flag, LoopState *st, bool from_acc = false) {
     if (is_done(st)) return;
-    __shared__ double red[kFinalizeCols / 32];
+    __shared__ double red[kFinalizeThreads / 32];
+    __shared__ long long part[3][kFinalizeThreads];
     const int j = blockIdx.x;
-    const int t = blockIdx.y * kFinalizeCols + threadIdx.x;
+    int dl, rp;  // column lanes, and threads per column
+    row_layout(min(d, kFinalizeCols), (int)blockDim.x, dl, rp);
+    const int rr = threadIdx.x / dl;
+    const int t = blockIdx.y * kFinalizeCols + threadIdx.x % dl;
     // from_acc: the maintained limb sums and counts hold this pass's sums in both
     // modes (the CSR form accumulates full passes there too)
     const bool full = !from_acc && st->upd_mode == 0;
     const long long c_j = full ? (long long)counts_sort[j] : cnt[j];
     double acc = 0.0;
-    if (t < d) {
-        const int64_t idx = (int64_t)j * d + t, plane = (int64_t)k * d, rplane = max_pieces * (int64_t)d;
-        long long s0 = 0, s1 = 0, s2 = 0;
-        if (full) {
-            for (int64_t p = piece_base[j]; p < piece_base[j + 1]; ++p) {
+    const int64_t idx = (int64_t)j * d + t, plane = (int64_t)k * d, rplane = max_pieces * (int64_t)d;
+    long long s0 = 0, s1 = 0, s2 = 0;
+    if (full) {  // the column's threads take every rp-th piece (integers: any order)
+        if (t < d) {
+#pragma unroll 4
+            for (int64_t p = piece_base[j] + rr; p < piece_base[j + 1]; p += rp) {
                 s0 += records[p * d + t];
                 s1 += records[rplane + p * d + t];
                 s2 += records[2 * rplane + p * d + t];
             }
-        } else {
+        }
+        part[0][threadIdx.x] = s0;
+        part[1][threadIdx.x] = s1;
+        part[2][threadIdx.x] = s2;
+        __syncthreads();
+        if (rr == 0)
+            for (int q = 1; q < rp; ++q) {
+                s0 += part[0][q * dl + threadIdx.x];
+                s1 += part[1][q * dl + threadIdx.x];
+                s2 += part[2][q * dl + threadIdx.x];
+            }
+    }
+    if (t < d && rr == 0) {
+        if (!full) {
             s0 = lacc[idx];
             s1 = lacc[plane + idx];
             s2 = lacc[2 * plane + idx];
@@ -1171,7 +1236,7 @@ finalize_exact_kernel(const long long *__restrict__ records, int64_t max_pieces,
     __syncthreads();
     if (threadIdx.x == 0) {
         double tot = 0.0;
-        for (int w = 0; w < kFinalizeCols / 32; ++w) tot += red[w];
+        for (int w = 0; w < (int)(blockDim.x / 32); ++w) tot += red[w];
         shift_tiles[(int64_t)j * gridDim.y + blockIdx.y] = tot;
         if (blockIdx.y == 0) {
             empty_flag[j] = c_j > 0 ? 0 : 1;
@@ -1560,7 +1625,7 @@ void launch_update_exact(const float *X, const UpdatePlan &p, int32_t *labels, c
     KMB_LAUNCHED();
     int32_t *empty_flag = (int32_t *)ws.empty_flag.ptr;
     const int tiles = (d + kFinalizeCols - 1) / kFinalizeCols;
-    finalize_exact_kernel<<<dim3((unsigned)k, (unsigned)tiles), kFinalizeCols, 0, s>>>(
+    finalize_exact_kernel<<<dim3((unsigned)k, (unsigned)tiles), kFinalizeThreads, 0, s>>>(
         records, p.max_pieces, (const int64_t *)ws.counts.ptr, (const int64_t *)ws.piece_base.ptr, colexp, k, acc,
         cnt, C_old, C_new, d, (double *)ws.shift_tiles.ptr, empty_flag, st);
     KMB_LAUNCHED();
@@ -1626,9 +1691,24 @@ void launch_partial_sums(const F *X, const UpdatePlan &p, const int32_t *labels,
 template <typename F>
 void launch_objective(const F *X, int64_t n, int64_t d, const F *C, const int32_t *labels, double *partials,
                       double *out, cudaStream_t s) {
-    objective_kernel<F><<<kObjectivePartials, 256, 0, s>>>(X, n, (int)d, C, labels, partials);
+    constexpr int V = 16 / (int)sizeof(F);
+    const uintptr_t both = (uintptr_t)X | (uintptr_t)C;
+    const int w = d % V == 0 && both % 16 == 0 ? V : (V == 4 && d % 2 == 0 && both % 8 == 0) ? 2 : 1;
+    auto launch = [&](auto w_tag, auto l_tag) {
+        objective_kernel<F, decltype(w_tag)::value, decltype(l_tag)::value>
+            <<<kObjectivePartials, 256, 0, s>>>(X, n, (int)d, C, labels, partials);
+    };
+    auto lanes = [&](auto w_tag) {  // lanes a row: its vectors, 4 to 16
+        const int64_t vecs = (d + decltype(w_tag)::value - 1) / decltype(w_tag)::value;
+        if (vecs <= 4) launch(w_tag, std::integral_constant<int, 4>());
+        else if (vecs <= 8) launch(w_tag, std::integral_constant<int, 8>());
+        else launch(w_tag, std::integral_constant<int, 16>());
+    };
+    if (w == V) lanes(std::integral_constant<int, V>());
+    else if (w == 2) lanes(std::integral_constant<int, 2>());
+    else lanes(std::integral_constant<int, 1>());
     KMB_LAUNCHED();
-    sum_partials_kernel<<<1, 32, 0, s>>>(partials, kObjectivePartials, out);
+    sum_partials_kernel<<<1, 256, 0, s>>>(partials, kObjectivePartials, out);
     KMB_LAUNCHED();
 }
 
@@ -1651,7 +1731,7 @@ template <typename F>
 void launch_sum_values(const F *v, int64_t n, double *partials, double *out, cudaStream_t s) {
     sum_values_kernel<F><<<kObjectivePartials, 256, 0, s>>>(v, n, partials);
     KMB_LAUNCHED();
-    sum_partials_kernel<<<1, 32, 0, s>>>(partials, kObjectivePartials, out);
+    sum_partials_kernel<<<1, 256, 0, s>>>(partials, kObjectivePartials, out);
     KMB_LAUNCHED();
 }
 
