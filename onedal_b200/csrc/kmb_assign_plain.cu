@@ -5,9 +5,15 @@
 //   argmin scan over clusters
 // (cpp/daal/src/algorithms/kmeans/kmeans_lloyd_impl.i:174-216 in the update loop and
 //  cpp/daal/src/algorithms/kmeans/kmeans_lloyd_postprocessing.h:95-130 for the final
-//  responses). The n x k score matrix is never materialised: each CTA owns a
-// 128-row tile, streams 128-cluster tiles of C^T through shared memory and keeps
-// a running (best, index, second, index2, third) per row in registers.
+//  responses). The n x k score matrix is never materialised: every kernel here streams
+// clusters past its rows and keeps a running best (with a recheck queue: best, second and
+// third) per row in registers.
+//
+//   assign_small_kernel     k <= 32 and d <= 64: a row per thread
+//   assign_f64_kernel       other double rows: FP64 on the tensor pipe
+//   assign_resident_kernel  float rows, many of them, clusters a multiple of 256 that fit
+//                           shared memory
+//   assign_few_kernel       all other float rows
 //
 // Scores are h_j - x.c_j with h_j = 0.5 ||c_j||^2 (the DAAL form); ties resolve to
 // the lowest cluster index. Rows whose best/second gap lies inside the derived
@@ -18,15 +24,14 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 namespace kmb {
 namespace {
 
-constexpr int BM = 128;  // rows per CTA
-constexpr int BN = 128;  // clusters per N-tile
-constexpr int BK = 8;    // contraction chunk
-constexpr int NT = 256;  // threads
-constexpr int PAD = 4;   // smem row padding (keeps 16-byte alignment, breaks bank conflicts)
+constexpr int BM = 128;  // rows per CTA (FP64)
+constexpr int BK = 8;    // columns that C^T's rows are padded to; the FP64 contraction chunk
+constexpr int NT = 256;  // threads (FP64)
 
 template <typename F> struct Vec4;
 template <> struct Vec4<float> { using T = float4; };
@@ -44,29 +49,6 @@ template <> __device__ __forceinline__ double unit_roundoff<double>() { return 1
 template <typename F>
 __device__ __forceinline__ bool lex_less(F a, int ia, F b, int ib) {
     return a < b || (a == b && ia < ib);
-}
-
-// acc[i][j] += a[i] * b[j] for the thread's 8 x 8 tile; for float as packed
-// pairs (fma.rn.f32x2: two correctly rounded FMAs, the same results as fmaf).
-template <typename F>
-__device__ __forceinline__ void fma_tile(F (&acc)[8][8], const F (&a)[8], const F (&b)[8]) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = fma(a[i], b[j], acc[i][j]);
-}
-template <>
-__device__ __forceinline__ void fma_tile<float>(float (&acc)[8][8], const float (&a)[8], const float (&b)[8]) {
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float2 ai = make_float2(a[i], a[i]);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const float2 t = __ffma2_rn(ai, make_float2(b[2 * q], b[2 * q + 1]), make_float2(acc[i][2 * q], acc[i][2 * q + 1]));
-            acc[i][2 * q] = t.x;
-            acc[i][2 * q + 1] = t.y;
-        }
-    }
 }
 
 template <typename F>
@@ -105,38 +87,8 @@ __device__ __forceinline__ void top_push_sel(RowTop<F> &r, F v, int c) {
     r.ib = lb ? c : r.ib;
 }
 
-template <typename F>
-__device__ __forceinline__ RowTop<F> top_merge(const RowTop<F> &x, const RowTop<F> &y) {
-    // Merge two sorted triples ((value, index) order); indices are kept for the
-    // first two places only. After o outputs a + b == o <= 2, so a, b < 3.
-    const F xv[3] = {x.b, x.s, x.t}, yv[3] = {y.b, y.s, y.t};
-    const int xi[3] = {x.ib, x.is, 0x7fffffff}, yi[3] = {y.ib, y.is, 0x7fffffff};
-    F ov[3];
-    int oi[3];
-    int a = 0, b = 0;
-#pragma unroll
-    for (int o = 0; o < 3; ++o) {
-        if (lex_less(xv[a], xi[a], yv[b], yi[b])) {
-            ov[o] = xv[a];
-            oi[o] = xi[a];
-            ++a;
-        } else {
-            ov[o] = yv[b];
-            oi[o] = yi[b];
-            ++b;
-        }
-    }
-    RowTop<F> r;
-    r.b = ov[0];
-    r.ib = oi[0];
-    r.s = ov[1];
-    r.is = oi[1];
-    r.t = ov[2];
-    return r;
-}
-
-// top_merge with selects instead of indexed arrays (the same result, the same
-// comparisons in the same argument order).
+// Merge of two sorted triples in (value, index) order, by selects; indices are kept for
+// the first two places only.
 template <typename F>
 __device__ __forceinline__ RowTop<F> top_merge_sel(const RowTop<F> &x, const RowTop<F> &y) {
     constexpr int kNone = 0x7fffffff;  // index of a third place
@@ -170,141 +122,364 @@ __device__ __forceinline__ RowTop<F> shfl_top(const RowTop<F> &x, int mask) {
     return y;
 }
 
-// float: two CTAs per SM (16 warps): the register cap of 128 costs a few spilled
-// epilogue values but doubles the warps that hide the FMA and shared-memory
-// latencies (10 % faster at d=128, k=1024 and 32 % at d=64, k=256).
-// double: one CTA per SM. The 8 x 8 FP64 accumulators alone take 128 registers;
-// under the 128 cap they spilled 3.5 KB per thread and ran at 2.9 TFLOP/s, with
-// 254 registers the same launch runs at 15.4 TFLOP/s (d=128, k=1024).
-template <typename F, bool VEC>
-__global__ void __launch_bounds__(NT, sizeof(F) == 4 ? 2 : 1)
-assign_plain_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restrict__ Ct, const F *__restrict__ h,
-                    int k, int kpad, const F *__restrict__ xnorm, const double *__restrict__ cnorm_max,
-                    int32_t *__restrict__ labels, F *__restrict__ d2, RecheckEntry *__restrict__ queue,
-                    LoopState *__restrict__ st) {
-    if (st && st->done) return;
-    using V4 = typename Vec4<F>::T;
-    __shared__ __align__(16) F Xs[2][BK][BM + PAD];
-    __shared__ __align__(16) F Cs[2][BK][BN + PAD];
-
-    const int tid = threadIdx.x;
-    const int ty = tid >> 4, tx = tid & 15;
-    const int64_t row0 = (int64_t)blockIdx.x * BM;
-
-    // Global-load mapping. X tile: 128 rows x 8 dims; thread -> row tid/2, dims (tid&1)*4..+3.
-    const int lr = tid >> 1, lk = (tid & 1) * 4;
-    const int64_t grow = row0 + lr;
-    const bool row_ok = grow < n;
-    const F *xrow = X + (row_ok ? grow : 0) * (int64_t)d;
-    // C tile: 8 dims x 128 clusters; thread -> dim tid/32, clusters (tid&31)*4..+3.
-    const int ck = tid >> 5, cn = (tid & 31) * 4;
-
-    const int nk = (d + BK - 1) / BK;
-    const int ntiles = kpad / BN;
-    const int steps = nk * ntiles;
-
-    F xr[4];
-    V4 cr;
-    auto gload = [&](int step) {
-        const int nt = step / nk, kc = step - nt * nk;
-        const int kb = kc * BK;
-        if (VEC) {
-            if (row_ok && kb + lk < d) {
-                V4 v = *reinterpret_cast<const V4 *>(xrow + kb + lk);
-                xr[0] = v.x; xr[1] = v.y; xr[2] = v.z; xr[3] = v.w;
-            } else {
-                xr[0] = xr[1] = xr[2] = xr[3] = F(0);
-            }
-        } else {
+// Keeps the rows of one half of `t` (hi: the upper half) and merges in the
+// partner lane's triples of the same rows.
+template <int R>
+__device__ __forceinline__ void res_exchange(RowTop<float> (&t)[8], int mask, bool hi) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) xr[q] = (row_ok && kb + lk + q < d) ? xrow[kb + lk + q] : F(0);
-        }
-        // Ct has nk*BK rows (zero padded) and kpad columns.
-        cr = *reinterpret_cast<const V4 *>(Ct + (int64_t)(kb + ck) * kpad + nt * BN + cn);
-    };
-    auto sstore = [&](int buf) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q) Xs[buf][lk + q][lr] = xr[q];
-        *reinterpret_cast<V4 *>(&Cs[buf][ck][cn]) = cr;
-    };
-
-    RowTop<F> top[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        top[i].b = top[i].s = top[i].t = f_inf<F>();
-        top[i].ib = 0;
-        top[i].is = 0;
+    for (int q = 0; q < R / 2; ++q) {
+        const RowTop<float> keep = hi ? t[R / 2 + q] : t[q];
+        const RowTop<float> send = hi ? t[q] : t[R / 2 + q];
+        t[q] = top_merge_sel(keep, shfl_top(send, mask));
     }
-    F acc[8][8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = F(0);
+}
 
-    gload(0);
-    sstore(0);
-    __syncthreads();
-
-    for (int step = 0; step < steps; ++step) {
-        const int buf = step & 1;
-        if (step + 1 < steps) gload(step + 1);
+// The best alone (value, lowest index): the same exchange.
+struct RowBest {
+    float b;
+    int ib;
+};
+__device__ __forceinline__ RowBest best_of(const RowBest &x, const RowBest &y) {
+    const bool c = lex_less(x.b, x.ib, y.b, y.ib);
+    return RowBest{c ? x.b : y.b, c ? x.ib : y.ib};
+}
+__device__ __forceinline__ RowBest shfl_best(const RowBest &x, int mask) {
+    return RowBest{__shfl_xor_sync(0xffffffffu, x.b, mask), __shfl_xor_sync(0xffffffffu, x.ib, mask)};
+}
+template <int R>
+__device__ __forceinline__ void best_exchange(RowBest (&t)[8], int mask, bool hi) {
 #pragma unroll
-        for (int kk = 0; kk < BK; ++kk) {
-            F a[8], b[8];
-            V4 a0 = *reinterpret_cast<const V4 *>(&Xs[buf][kk][ty * 4]);
-            V4 a1 = *reinterpret_cast<const V4 *>(&Xs[buf][kk][64 + ty * 4]);
-            V4 b0 = *reinterpret_cast<const V4 *>(&Cs[buf][kk][tx * 4]);
-            V4 b1 = *reinterpret_cast<const V4 *>(&Cs[buf][kk][64 + tx * 4]);
-            a[0] = a0.x; a[1] = a0.y; a[2] = a0.z; a[3] = a0.w;
-            a[4] = a1.x; a[5] = a1.y; a[6] = a1.z; a[7] = a1.w;
-            b[0] = b0.x; b[1] = b0.y; b[2] = b0.z; b[3] = b0.w;
-            b[4] = b1.x; b[5] = b1.y; b[6] = b1.z; b[7] = b1.w;
-            fma_tile(acc, a, b);
+    for (int q = 0; q < R / 2; ++q) {
+        const RowBest keep = hi ? t[R / 2 + q] : t[q];
+        const RowBest send = hi ? t[q] : t[R / 2 + q];
+        t[q] = best_of(keep, shfl_best(send, mask));
+    }
+}
+
+__device__ __forceinline__ void cp_async_zfill(void *smem, const void *gmem, int bytes, bool ok) {
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    if (bytes == 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(s), "l"(gmem), "r"(ok ? 4 : 0) : "memory");
+    else if (bytes == 8)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(s), "l"(gmem), "r"(ok ? 8 : 0) : "memory");
+    else
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(s), "l"(gmem), "r"(ok ? 16 : 0) : "memory");
+}
+
+// ---- float rows --------------------------------------------------------------
+// 32 rows per CTA (so a few thousand rows already cover the SMs): 4 warps of 8 rows, a
+// lane the clusters 4l .. 4l+3 and 128+4l .. of each 256-cluster pass (the first four alone
+// where a pass holds 128); row values are shared-memory broadcasts, centroid chunks of 16
+// columns come by cp.async in a ring of two. Dot products add x_t * c_t in ascending t with
+// FMAs from zero: the scores, and the labels, distances and recheck entries, are those of
+// the other float kernels. Without a queue only a row's best is kept (a compare and two
+// selects per score instead of ten instructions). Bound by the operands' way from shared
+// memory into registers, one byte per FMA. Per launch, against the kernels used before (128
+// x 128 tiles per CTA; 64-row tiles with resident centroids):
+//   4097 x 64, k = 300 40 -> 11.6 us; 76,000 x 64, k = 300 173 -> 105; 300,000 x 128, k =
+//   1000 2018 -> 1724; 1M x 37, k = 300 1295 -> 979; 50,000 x 1000, k = 500 1855 -> 1150
+constexpr int kFewRows = 32, kFewPass = 256, kFewK = 16, kFewThreads = 128, kFewR = 8;
+
+template <bool VEC, bool TOP3>
+__global__ void __launch_bounds__(kFewThreads, 3)
+assign_few_kernel(const float *__restrict__ X, int64_t n, int d, const float *__restrict__ Ct,
+                  const float *__restrict__ h, int k, int kpad, const float *__restrict__ xnorm,
+                  const double *__restrict__ cnorm_max, int32_t *__restrict__ labels, float *__restrict__ d2,
+                  RecheckEntry *__restrict__ queue, LoopState *__restrict__ st) {
+    if (st && st->done) return;
+    __shared__ __align__(16) float Xs[2][kFewRows][kFewK];
+    __shared__ __align__(16) float Cs[2][kFewK][kFewPass];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t row0 = (int64_t)blockIdx.x * kFewRows;
+    const int dpad = (d + BK - 1) / BK * BK;           // rows of Ct
+    const int nk = (d + kFewK - 1) / kFewK;
+    const int npass = (kpad + kFewPass - 1) / kFewPass;
+    const int steps = nk * npass;
+    auto issue = [&](int step) {
+        if (step < steps) {
+            const int ps = step / nk, kb = (step - ps * nk) * kFewK, buf = step & 1;
+            if (tid < kFewRows * kFewK / 4) {  // a row's four columns a thread
+                const int r = tid / (kFewK / 4), c = 4 * (tid % (kFewK / 4));
+                const float *src = X + (row0 + r < n ? row0 + r : 0) * d + kb + c;
+                if (VEC) {  // d % 4 == 0 at a 16-byte aligned base
+                    const bool ok = row0 + r < n && kb + c < d;
+                    cp_async_zfill(&Xs[buf][r][c], ok ? src : X, 16, ok);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const bool ok = row0 + r < n && kb + c + i < d;
+                        cp_async_zfill(&Xs[buf][r][c + i], ok ? src + i : X, 4, ok);
+                    }
+                }
+            }
+#pragma unroll
+            for (int i = 0; i < kFewK * kFewPass / 4 / kFewThreads; ++i) {
+                const int e = tid + i * kFewThreads, r = e / (kFewPass / 4), c = 4 * (e % (kFewPass / 4));
+                const bool ok = kb + r < dpad && ps * kFewPass + c < kpad;
+                cp_async_zfill(&Cs[buf][r][c], ok ? Ct + (int64_t)(kb + r) * kpad + ps * kFewPass + c : Ct, 16, ok);
+            }
         }
-        const int nt = step / nk;
-        if (step - nt * nk == nk - 1) {
-            // Epilogue of one N-tile: scores h_j - x.c_j into the running top-3.
-            const int cbase = nt * BN;
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    RowTop<float> top[TOP3 ? kFewR : 1];  // TOP3: for the recheck queue; else the best alone
+    RowBest best[TOP3 ? 1 : kFewR];
+    float2 acc[kFewR][4];  // acc[i][q]: clusters 2q, 2q + 1 of this lane's eight
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const int col = cbase + (j < 4 ? tx * 4 + j : 64 + tx * 4 + (j - 4));
-                const F hj = h[col];
+    for (int i = 0; i < kFewR; ++i) {
+        if constexpr (TOP3) {
+            top[i].b = top[i].s = top[i].t = f_inf<float>();
+            top[i].ib = top[i].is = 0;
+        } else {
+            best[i] = RowBest{f_inf<float>(), 0};
+        }
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    top_push_sel(top[i], hj - acc[i][j], col);
-                    acc[i][j] = F(0);
+        for (int q = 0; q < 4; ++q) acc[i][q] = make_float2(0.f, 0.f);
+    }
+    issue(0);
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncthreads();  // the step's chunks are visible, and every warp is done with the other buffer
+        issue(step + 1);
+        const int buf = step & 1, ps = step / nk;
+        auto contract = [&](auto q_tag) {  // Q pairs of this lane's clusters
+            constexpr int Q = decltype(q_tag)::value;
+#pragma unroll
+            for (int t = 0; t < kFewK; t += 2) {
+                float2 a[kFewR];
+#pragma unroll
+                for (int i = 0; i < kFewR; ++i) a[i] = *reinterpret_cast<const float2 *>(&Xs[buf][kFewR * warp + i][t]);
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const float4 b0 = *reinterpret_cast<const float4 *>(&Cs[buf][t + u][4 * lane]);
+                    float2 b[Q];
+                    b[0] = make_float2(b0.x, b0.y);
+                    b[1] = make_float2(b0.z, b0.w);
+                    if constexpr (Q == 4) {
+                        const float4 b1 = *reinterpret_cast<const float4 *>(&Cs[buf][t + u][128 + 4 * lane]);
+                        b[2] = make_float2(b1.x, b1.y);
+                        b[3] = make_float2(b1.z, b1.w);
+                    }
+#pragma unroll
+                    for (int i = 0; i < kFewR; ++i) {
+                        const float x = u ? a[i].y : a[i].x;
+#pragma unroll
+                        for (int q = 0; q < Q; ++q) acc[i][q] = __ffma2_rn(make_float2(x, x), b[q], acc[i][q]);
+                    }
+                }
+            }
+        };
+        const bool narrow = ps * kFewPass + 128 >= kpad;
+        if (narrow) contract(std::integral_constant<int, 2>());
+        else contract(std::integral_constant<int, 4>());
+        if (step - ps * nk == nk - 1) {  // the pass's scores, this lane's clusters in ascending order
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if (q >= 2 && narrow) break;
+                const int col = ps * kFewPass + (q < 2 ? 4 * lane + 2 * q : 124 + 4 * lane + 2 * q);
+                const float h0 = col < kpad ? h[col] : f_inf<float>(), h1 = col + 1 < kpad ? h[col + 1] : f_inf<float>();
+#pragma unroll
+                for (int i = 0; i < kFewR; ++i) {
+                    const float v0 = h0 - acc[i][q].x, v1 = h1 - acc[i][q].y;
+                    if constexpr (TOP3) {
+                        top_push_sel(top[i], v0, col);
+                        top_push_sel(top[i], v1, col + 1);
+                    } else {
+                        best[i].ib = v0 < best[i].b ? col : best[i].ib;
+                        best[i].b = v0 < best[i].b ? v0 : best[i].b;
+                        best[i].ib = v1 < best[i].b ? col + 1 : best[i].ib;
+                        best[i].b = v1 < best[i].b ? v1 : best[i].b;
+                    }
+                    acc[i][q] = make_float2(0.f, 0.f);
                 }
             }
         }
-        if (step + 1 < steps) sstore(buf ^ 1);
-        __syncthreads();
     }
-
-    // Reduce across the 16 lanes (tx) that share the same rows.
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-#pragma unroll
-        for (int m = 8; m >= 1; m >>= 1) top[i] = top_merge_sel(top[i], shfl_top(top[i], m));
+    // lanes exchange halves of their rows; row `own` ends in four lanes
+    const bool h16 = (lane >> 4) & 1, h8 = (lane >> 3) & 1, h4 = (lane >> 2) & 1;
+    const int own = 4 * h16 + 2 * h8 + h4;
+    if constexpr (TOP3) {
+        res_exchange<8>(top, 16, h16);
+        res_exchange<4>(top, 8, h8);
+        res_exchange<2>(top, 4, h4);
+        top[0] = top_merge_sel(top[0], shfl_top(top[0], 2));
+        top[0] = top_merge_sel(top[0], shfl_top(top[0], 1));
+    } else {
+        best_exchange<8>(best, 16, h16);
+        best_exchange<4>(best, 8, h8);
+        best_exchange<2>(best, 4, h4);
+        best[0] = best_of(best[0], shfl_best(best[0], 2));
+        best[0] = best_of(best[0], shfl_best(best[0], 1));
     }
-    if (tx == 0) {
-        const double u = unit_roundoff<F>();
-        const double cmax = cnorm_max ? *cnorm_max : 0.0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int64_t r = row0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
-            if (r >= n) continue;
-            const RowTop<F> &t = top[i];
+    if ((lane & 3) == 0) {
+        RowTop<float> t = {};
+        if constexpr (TOP3) {
+            t = top[0];
+        } else {
+            t.b = best[0].b;
+            t.ib = best[0].ib;
+        }
+        const int64_t r = row0 + kFewR * warp + own;
+        if (r < n) {
             labels[r] = t.ib;
-            const F xn = xnorm[r];
-            d2[r] = F(2) * t.b + xn;
-            if (queue) {
-                // |computed - exact| per score <= u*cmax^2 + (d+2)*u*||x||*cmax (+ slack);
-                // the order of two scores is certain when their gap exceeds twice that.
+            const float xn = xnorm[r];
+            d2[r] = 2.0f * t.b + xn;
+            if (TOP3 && queue) {
+                const double cmax = cnorm_max ? *cnorm_max : 0.0;
                 const double xl = sqrt(fmax((double)xn, 0.0));
-                const double e = 1.0625 * u * (cmax * cmax + (double)(d + 2) * xl * cmax);
+                const double e = 1.0625 * unit_roundoff<float>() * (cmax * cmax + (double)(d + 2) * xl * cmax);
                 const double band = 2.0 * e;
                 if ((double)t.s - (double)t.b <= band)
                     enqueue_recheck(queue, n, st, (int)r, t.ib, t.is, (double)t.t - (double)t.b <= band);
+            }
+        }
+    }
+}
+
+// ---- FP64 on the tensor pipe --------------------------------------------------
+// Double rows: a CTA of 8 warps (4 x 2) scores 128 rows against tiles of BN clusters with
+// mma.sync m8n8k4.f64, whose products and sums are FP64 FMAs (the FP64 rate of the tensor
+// pipe is that of the FMA pipe here, but a warp's 32 x BN/2 tile takes 12 operand values
+// from shared memory for 256 FMAs per lane where the 8 x 8 tile per thread took 16 for 64:
+// its shared-memory reads bounded it). Row and centroid chunks of 8 columns arrive by
+// cp.async in a ring of three; the pitches (12 and BN + 4 doubles) keep the 8-byte fragment
+// reads free of bank conflicts. BN = 64 where it pads k less than 128 does. TOP3: the
+// running third place is kept for the recheck queue; else the best alone.
+// Per launch: 300,007 x 37, k = 101 349 -> 179 us; 500,000 x 128, k = 1024 8.18 -> 5.03 ms
+// (26 TFLOP/s).
+constexpr int kDP = BK + 4;  // row pitch of the staged X chunk, in doubles
+constexpr int kDStages = 3;
+
+__device__ __forceinline__ void dmma(double (&c)[2], double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(c[0]), "+d"(c[1])
+                 : "d"(a), "d"(b));
+}
+
+template <int BNT>
+constexpr size_t f64_smem_bytes() { return sizeof(double) * kDStages * (BM * kDP + BK * (BNT + 4)); }
+
+template <int BNT, bool TOP3>
+__global__ void __launch_bounds__(NT, 1)
+assign_f64_kernel(const double *__restrict__ X, int64_t n, int d, const double *__restrict__ Ct,
+                  const double *__restrict__ h, int k, int kpad, const double *__restrict__ xnorm,
+                  const double *__restrict__ cnorm_max, int32_t *__restrict__ labels, double *__restrict__ d2,
+                  RecheckEntry *__restrict__ queue, LoopState *__restrict__ st) {
+    if (st && st->done) return;
+    constexpr int CP = BNT + 4;     // pitch of the staged centroid chunk
+    constexpr int NTL = BNT / 16;   // 8-cluster tiles of a warp
+    extern __shared__ __align__(16) double f64_smem[];
+    double *Xs = f64_smem, *Cs = f64_smem + kDStages * BM * kDP;
+    __shared__ RowTop<double> s_top[BM];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int wr = warp & 3, wc = warp >> 2;  // rows 32 wr .., clusters BNT/2 wc ..
+    const int g = lane >> 2, q4 = lane & 3;
+    const int64_t row0 = (int64_t)blockIdx.x * BM;
+    const int nk = (d + BK - 1) / BK;
+    const int ntiles = (k + BNT - 1) / BNT;  // (tiles of padding alone are left out)
+    const int steps = nk * ntiles;
+    auto issue = [&](int step) {
+        if (step < steps) {
+            const int nt = step / nk, kb = (step - nt * nk) * BK, stage = step % kDStages;
+            double *xd = Xs + stage * BM * kDP, *cd = Cs + stage * BK * CP;
+#pragma unroll
+            for (int i = 0; i < BM * BK / NT; ++i) {
+                const int e = tid + i * NT, r = e / BK, c = e % BK;
+                const bool ok = row0 + r < n && kb + c < d;
+                cp_async_zfill(xd + r * kDP + c, ok ? X + (row0 + r) * d + kb + c : X, 8, ok);
+            }
+#pragma unroll
+            for (int i = 0; i < BK * BNT / 2 / NT; ++i) {  // Ct has nk * BK rows, kpad columns (a multiple of 128)
+                const int e = tid + i * NT, r = e / (BNT / 2), c = 2 * (e % (BNT / 2));
+                cp_async_zfill(cd + r * CP + c, Ct + (int64_t)(kb + r) * kpad + nt * BNT + c, 16, true);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    RowTop<double> top[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        top[i].b = top[i].s = top[i].t = f_inf<double>();
+        top[i].ib = top[i].is = 0;
+    }
+    double acc[4][NTL][2];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < NTL; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+    for (int p = 0; p < kDStages - 1; ++p) issue(p);
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(kDStages - 2) : "memory");
+        __syncthreads();  // the step's chunks are visible, and every warp is done with the oldest stage
+        issue(step + kDStages - 1);
+        const int stage = step % kDStages;
+        const double *xs = Xs + stage * BM * kDP + (32 * wr + g) * kDP + q4;
+        const double *cs = Cs + stage * BK * CP + q4 * CP + wc * (BNT / 2) + g;
+#pragma unroll
+        for (int kk = 0; kk < BK; kk += 4) {
+            double a[4], b[NTL];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i] = xs[8 * i * kDP + kk];
+#pragma unroll
+            for (int j = 0; j < NTL; ++j) b[j] = cs[kk * CP + 8 * j];
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int j = 0; j < NTL; ++j) dmma(acc[i][j], a[i], b[j]);
+        }
+        const int nt = step / nk;
+        if (step - nt * nk == nk - 1) {  // the tile's scores h_j - x.c_j into the running places
+            const int col0 = nt * BNT + wc * (BNT / 2) + 2 * q4;
+#pragma unroll
+            for (int j = 0; j < NTL; ++j) {
+                const int col = col0 + 8 * j;
+                const double h0 = h[col], h1 = h[col + 1];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const double v0 = h0 - acc[i][j][0], v1 = h1 - acc[i][j][1];
+                    acc[i][j][0] = acc[i][j][1] = 0.0;
+                    if constexpr (TOP3) {
+                        top_push_sel(top[i], v0, col);
+                        top_push_sel(top[i], v1, col + 1);
+                    } else {
+                        if (v0 < top[i].b) {
+                            top[i].b = v0;
+                            top[i].ib = col;
+                        }
+                        if (v1 < top[i].b) {
+                            top[i].b = v1;
+                            top[i].ib = col + 1;
+                        }
+                    }
+                }
+            }
+        }
+    }
+    // a row's places from its four lanes, then from the two warps that share it
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        top[i] = top_merge_sel(top[i], shfl_top(top[i], 1));
+        top[i] = top_merge_sel(top[i], shfl_top(top[i], 2));
+        if (wc == 1 && q4 == 0) s_top[32 * wr + 8 * i + g] = top[i];
+    }
+    __syncthreads();
+    if (wc == 0 && q4 == 0) {
+        const double u = unit_roundoff<double>();
+        const double cmax = cnorm_max ? *cnorm_max : 0.0;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int64_t r = row0 + 32 * wr + 8 * i + g;
+            if (r >= n) continue;
+            const RowTop<double> t = top_merge_sel(top[i], s_top[32 * wr + 8 * i + g]);
+            labels[r] = t.ib;
+            const double xn = xnorm[r];
+            d2[r] = 2.0 * t.b + xn;
+            if (TOP3 && queue) {
+                // |computed - exact| per score <= u*cmax^2 + (d+2)*u*||x||*cmax (+ slack), in any
+                // order of the FMAs; two scores further apart than twice that are in order
+                const double xl = sqrt(fmax(xn, 0.0));
+                const double e = 1.0625 * u * (cmax * cmax + (double)(d + 2) * xl * cmax);
+                const double band = 2.0 * e;
+                if (t.s - t.b <= band) enqueue_recheck(queue, n, st, (int)r, t.ib, t.is, t.t - t.b <= band);
             }
         }
     }
@@ -359,7 +534,7 @@ constexpr int kSmallThreads = 128;
 
 // Few clusters (k <= 32, d <= 64): one row per thread, its d values in registers,
 // all centroids in shared memory (read as broadcasts). The contraction of row and
-// cluster accumulates x_t * c_t in ascending t, as the tiled kernel does, so the
+// cluster accumulates x_t * c_t in ascending t, as the other kernels do, so the
 // scores -- and the labels, distances and recheck entries -- are the same; only
 // the 128-cluster tile padding and the tile epilogue are gone.
 template <typename F, int DMAX>
@@ -422,9 +597,10 @@ assign_small_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restri
 // 4l..4l+3 and 128+4l..128+4l+3 of each 256-cluster pass: the row values are
 // shared-memory broadcasts and the centroid reads are conflict-free 16-byte
 // loads. Per (row, cluster) the contraction accumulates x_t * c_t in ascending
-// t with FMAs from zero, as assign_plain_kernel does, so the scores -- and the
+// t with FMAs from zero, as the other float kernels do, so the scores -- and the
 // labels, distances and recheck entries -- are the same. After each pass a
-// lane holds the top-3 of its 8 clusters for its warp's 8 rows; five exchange
+// lane holds the top-3 (the best alone without a recheck queue: 10M x 64, k = 256 8.62 ms
+// a launch with the top-3, 7.34 ms with the best) of its 8 clusters for its warp's 8 rows; five exchange
 // rounds halve the rows a lane keeps while merging in the partner's (value,
 // index) triples, leaving each row's top-3 in four lanes; with more than one
 // pass the row's owner lane merges it into the running top-3 in shared memory.
@@ -508,24 +684,12 @@ __device__ __forceinline__ void res_turn_give(int id) {
     asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(kResThreads) : "memory");
 }
 
-// Keeps the rows of one half of `t` (hi: the upper half) and merges in the
-// partner lane's triples of the same rows.
-template <int R>
-__device__ __forceinline__ void res_exchange(RowTop<float> (&t)[8], int mask, bool hi) {
-#pragma unroll
-    for (int q = 0; q < R / 2; ++q) {
-        const RowTop<float> keep = hi ? t[R / 2 + q] : t[q];
-        const RowTop<float> send = hi ? t[q] : t[R / 2 + q];
-        t[q] = top_merge_sel(keep, shfl_top(send, mask));
-    }
-}
-
 // DPADT > 0 fixes the padded row width at compile time (row and centroid offsets
 // become immediates); 0 reads it from dpad. STAGES: TMA stages per group (1 or 2).
 // kres: all clusters, padded to 256; kchunk: clusters resident at a time (kres when
 // n_chunks == 1); bt: row tiles per block and group (the running top-3 rows).
 // CHUNK false: all clusters resident (n_chunks = bt = 1 at compile time).
-template <int DPADT, int STAGES, bool CHUNK>
+template <int DPADT, int STAGES, bool CHUNK, bool TOP3>
 __global__ void __launch_bounds__(kResThreads, 1)
 assign_resident_kernel(const __grid_constant__ CUtensorMap tmX, int64_t n, int d, int dpad_rt, const float *__restrict__ Ct,
                        const float *__restrict__ h, int k, int kpad, int kres, int kchunk, int n_chunks_rt, int bt_rt,
@@ -720,26 +884,57 @@ assign_resident_kernel(const __grid_constant__ CUtensorMap tmX, int64_t n, int d
 #pragma unroll
                     for (int j = 0; j < 8; ++j) hv[j] = hs[pass * kResPass + (j < 4 ? 4 * lane + j : 128 + 4 * lane + (j - 4))];
                     const int col0 = c0 + pass * kResPass + 4 * lane;
-                    RowTop<float> top[8];
+                    RowTop<float> r = {};  // row `own`'s places, in four lanes after the exchange
+                    if constexpr (TOP3) {
+                        RowTop<float> top[8];
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) {
-                        const float v0 = hv[0] - acc[i][0];
-                        const bool l0 = v0 < f_inf<float>();  // a push into an empty triple
-                        top[i].b = l0 ? v0 : f_inf<float>();
-                        top[i].ib = l0 ? col0 : 0;
-                        top[i].s = top[i].t = f_inf<float>();
-                        top[i].is = 0;
+                        for (int i = 0; i < 8; ++i) {
+                            const float v0 = hv[0] - acc[i][0];
+                            const bool l0 = v0 < f_inf<float>();  // a push into an empty triple
+                            top[i].b = l0 ? v0 : f_inf<float>();
+                            top[i].ib = l0 ? col0 : 0;
+                            top[i].s = top[i].t = f_inf<float>();
+                            top[i].is = 0;
 #pragma unroll
-                        for (int j = 1; j < 8; ++j) top_push_sel(top[i], hv[j] - acc[i][j], col0 + (j < 4 ? j : 124 + j));
+                            for (int j = 1; j < 8; ++j) top_push_sel(top[i], hv[j] - acc[i][j], col0 + (j < 4 ? j : 124 + j));
+                        }
+                        res_exchange<8>(top, 16, (lane >> 4) & 1);
+                        res_exchange<4>(top, 8, (lane >> 3) & 1);
+                        res_exchange<2>(top, 4, (lane >> 2) & 1);
+                        top[0] = top_merge_sel(top[0], shfl_top(top[0], 2));
+                        top[0] = top_merge_sel(top[0], shfl_top(top[0], 1));
+                        r = top[0];
+                    } else {
+                        RowBest best[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            best[i] = RowBest{f_inf<float>(), 0};
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) {
+                                const float v = hv[j] - acc[i][j];
+                                const bool l = v < best[i].b;
+                                best[i].ib = l ? col0 + (j < 4 ? j : 124 + j) : best[i].ib;
+                                best[i].b = l ? v : best[i].b;
+                            }
+                        }
+                        best_exchange<8>(best, 16, (lane >> 4) & 1);
+                        best_exchange<4>(best, 8, (lane >> 3) & 1);
+                        best_exchange<2>(best, 4, (lane >> 2) & 1);
+                        best[0] = best_of(best[0], shfl_best(best[0], 2));
+                        best[0] = best_of(best[0], shfl_best(best[0], 1));
+                        r.b = best[0].b;
+                        r.ib = best[0].ib;
                     }
-                    res_exchange<8>(top, 16, (lane >> 4) & 1);
-                    res_exchange<4>(top, 8, (lane >> 3) & 1);
-                    res_exchange<2>(top, 4, (lane >> 2) & 1);
-                    top[0] = top_merge_sel(top[0], shfl_top(top[0], 2));
-                    top[0] = top_merge_sel(top[0], shfl_top(top[0], 1));
                     if ((lane & 3) == 0) {
-                        RowTop<float> r = top[0];
-                        if (q > 0 || pass > 0) r = top_merge_sel(grun[own], r);
+                        if (q > 0 || pass > 0) {
+                            if constexpr (TOP3) {
+                                r = top_merge_sel(grun[own], r);
+                            } else {
+                                const RowBest m = best_of(RowBest{grun[own].b, grun[own].ib}, RowBest{r.b, r.ib});
+                                r.b = m.b;
+                                r.ib = m.ib;
+                            }
+                        }
                         if (q + 1 < n_chunks || !last_pass) {
                             grun[own] = r;
                         } else {
@@ -748,7 +943,7 @@ assign_resident_kernel(const __grid_constant__ CUtensorMap tmX, int64_t n, int d
                                 labels[row] = r.ib;
                                 const float xn = xnorm[row];
                                 d2[row] = 2.0f * r.b + xn;
-                                if (queue) {
+                                if (TOP3 && queue) {
                                     const double xl = sqrt(fmax((double)xn, 0.0));
                                     const double e = 1.0625 * u * (cmax * cmax + (double)(d + 2) * xl * cmax);
                                     const double band = 2.0 * e;
@@ -832,8 +1027,15 @@ bool launch_resident<float>(const float *X, int64_t n, int64_t d, const float *C
                             RecheckEntry *queue, LoopState *st, cudaStream_t s) {
     if (d % 4 != 0 || d > 256 || (reinterpret_cast<uintptr_t>(X) % 16) != 0 || n > INT32_MAX - 2 * kResCtaRows)
         return false;
+    // KMB_PLAIN_RESIDENT: 0 never, 1 wherever it applies (tests compare the two); else the
+    // size rule below
     const char *e = getenv("KMB_PLAIN_RESIDENT");
     if (e && e[0] == '0') return false;
+    const bool forced = e && e[0] == '1';
+    // The better one for many rows and whole 256-cluster passes: 300,000 x 64, k = 256 241 us
+    // against 246, 3M 2236 against 2313 (76,000: 78 against 68; 3M x 64, k = 300, whose
+    // second pass is mostly padding here, 4422 against 3652)
+    if (!forced && (n < (1 << 18) || kpad % kResPass != 0)) return false;
     const int dpad = (int)((d + BK - 1) / BK * BK);  // the rows of Ct
     const int kres = (int)((kpad + kResPass - 1) / kResPass * kResPass);
     int dev = 0, optin = 0, sms = 148;
@@ -863,6 +1065,8 @@ bool launch_resident<float>(const float *X, int64_t n, int64_t d, const float *C
         kchunk = (kres / kResPass + nc - 1) / nc * kResPass;
     }
     const int n_chunks = (kres + kchunk - 1) / kchunk;
+    // (chunks: 300,000 x 128, k = 1000 1872 us against 1724, 3M 18.4 ms against 16.6)
+    if (!forced && n_chunks > 1) return false;
     const size_t smem = resident_smem_bytes(dpad, kchunk, stages, bt);
     if (smem > (size_t)optin) return false;
     CUtensorMap tm;
@@ -870,14 +1074,19 @@ bool launch_resident<float>(const float *X, int64_t n, int64_t d, const float *C
     if (!encode_tensor_map_2d(&tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, X, (uint64_t)d, (uint64_t)n, (uint64_t)d * 4,
                               (uint32_t)dpad, (uint32_t)kResRows, CU_TENSOR_MAP_SWIZZLE_NONE))
         return false;
-    auto pick = [&](auto k32, auto k64, auto k128, auto k0) { return dpad == 32 ? k32 : dpad == 64 ? k64 : dpad == 128 ? k128 : k0; };
-    auto kern = n_chunks == 1 && bt == 1
-                    ? pick(assign_resident_kernel<32, 2, false>, assign_resident_kernel<64, 2, false>,
-                           assign_resident_kernel<128, 2, false>, assign_resident_kernel<0, 2, false>)
-                : stages == 2 ? pick(assign_resident_kernel<32, 2, true>, assign_resident_kernel<64, 2, true>,
-                                     assign_resident_kernel<128, 2, true>, assign_resident_kernel<0, 2, true>)
-                              : pick(assign_resident_kernel<32, 1, true>, assign_resident_kernel<64, 1, true>,
-                                     assign_resident_kernel<128, 1, true>, assign_resident_kernel<0, 1, true>);
+    // without a recheck queue only the best cluster of a row is kept
+    auto pick = [&](auto top3) {
+        constexpr bool T3 = decltype(top3)::value;
+        auto by_d = [&](auto k32, auto k64, auto k128, auto k0) { return dpad == 32 ? k32 : dpad == 64 ? k64 : dpad == 128 ? k128 : k0; };
+        return n_chunks == 1 && bt == 1
+                   ? by_d(assign_resident_kernel<32, 2, false, T3>, assign_resident_kernel<64, 2, false, T3>,
+                          assign_resident_kernel<128, 2, false, T3>, assign_resident_kernel<0, 2, false, T3>)
+               : stages == 2 ? by_d(assign_resident_kernel<32, 2, true, T3>, assign_resident_kernel<64, 2, true, T3>,
+                                    assign_resident_kernel<128, 2, true, T3>, assign_resident_kernel<0, 2, true, T3>)
+                             : by_d(assign_resident_kernel<32, 1, true, T3>, assign_resident_kernel<64, 1, true, T3>,
+                                    assign_resident_kernel<128, 1, true, T3>, assign_resident_kernel<0, 1, true, T3>);
+    };
+    auto kern = queue ? pick(std::true_type()) : pick(std::false_type());
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
         cudaGetLastError();
         return false;
@@ -888,6 +1097,19 @@ bool launch_resident<float>(const float *X, int64_t n, int64_t d, const float *C
                                          xnorm, cnorm_max, labels, d2, queue, st);
     KMB_LAUNCHED();
     return true;
+}
+
+static void launch_f64(unsigned blocks, const double *X, int64_t n, int64_t d, const double *Ct, const double *h,
+                       int64_t k, int64_t kpad, const double *xnorm, const double *cnorm_max, int32_t *labels,
+                       double *d2, RecheckEntry *queue, LoopState *st, cudaStream_t s) {
+    // 64-cluster tiles where they pad k to fewer clusters
+    const bool narrow = (k + 63) / 64 * 64 < (k + 127) / 128 * 128;
+    auto kern = narrow ? (queue ? assign_f64_kernel<64, true> : assign_f64_kernel<64, false>)
+                       : (queue ? assign_f64_kernel<128, true> : assign_f64_kernel<128, false>);
+    const int smem = (int)(narrow ? f64_smem_bytes<64>() : f64_smem_bytes<128>());
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess) return;
+    kern<<<blocks, NT, smem, s>>>(X, n, (int)d, Ct, h, (int)k, (int)kpad, xnorm, cnorm_max, labels, d2, queue, st);
+    KMB_LAUNCHED();
 }
 
 template <typename F>
@@ -901,16 +1123,15 @@ void launch_assign_plain(const F *X, int64_t n, int64_t d, const F *Ct, const F 
         else launch_small<F, 64>(X, n, d, Ct, h, k, kpad, xnorm, cnorm_max, labels, d2, queue, st, s);
         return;
     }
-    if (launch_resident(X, n, d, Ct, h, k, kpad, xnorm, cnorm_max, labels, d2, queue, st, s)) return;
-    const unsigned blocks = (unsigned)((n + BM - 1) / BM);
-    const bool vec = (d % 4 == 0) && ((reinterpret_cast<uintptr_t>(X) % (4 * sizeof(F))) == 0);
-    if (vec) {
-        assign_plain_kernel<F, true><<<blocks, NT, 0, s>>>(X, n, (int)d, Ct, h, (int)k, (int)kpad, xnorm, cnorm_max,
-            labels, d2, queue, st);
-        KMB_LAUNCHED();
+    if constexpr (sizeof(F) == 8) {
+        launch_f64((unsigned)((n + BM - 1) / BM), X, n, d, Ct, h, k, kpad, xnorm, cnorm_max, labels, d2, queue, st, s);
     } else {
-        assign_plain_kernel<F, false><<<blocks, NT, 0, s>>>(X, n, (int)d, Ct, h, (int)k, (int)kpad, xnorm, cnorm_max,
-            labels, d2, queue, st);
+        if (launch_resident(X, n, d, Ct, h, k, kpad, xnorm, cnorm_max, labels, d2, queue, st, s)) return;
+        const bool vec = d % 4 == 0 && (reinterpret_cast<uintptr_t>(X) % 16) == 0;
+        auto kern = vec ? (queue ? assign_few_kernel<true, true> : assign_few_kernel<true, false>)
+                        : (queue ? assign_few_kernel<false, true> : assign_few_kernel<false, false>);
+        kern<<<(unsigned)((n + kFewRows - 1) / kFewRows), kFewThreads, 0, s>>>(X, n, (int)d, Ct, h, (int)k, (int)kpad,
+                                                                              xnorm, cnorm_max, labels, d2, queue, st);
         KMB_LAUNCHED();
     }
 }
