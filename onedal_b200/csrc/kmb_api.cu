@@ -285,8 +285,9 @@ int ensure_common(kmb_context *ctx, int64_t n, int64_t d, int64_t k, bool rechec
 }
 
 // Before a pass: its counters, and max ||c|| (the previous pass's kept in *cmax_prev
-// when given).
-__global__ void reset_iteration_kernel(LoopState *st, double *cmax, double *cmax_prev) {
+// when given). init: the whole state starts from zeros (a call of one pass).
+__global__ void reset_iteration_kernel(LoopState *st, double *cmax, double *cmax_prev, bool init) {
+    if (init) *st = LoopState();
     if (st->done) return;
     if (cmax_prev) *cmax_prev = *cmax;
     *cmax = 0.0;
@@ -305,17 +306,17 @@ __global__ void account_recheck_kernel(LoopState *st) {
 // One assignment pass of the plain form (+ optional FP64 recheck) under C.
 template <typename F>
 int assign_pass_tc(kmb_context *ctx, const F *X, int64_t n, int64_t d, const F *C, int64_t k, int32_t *labels,
-                   F *d2, LoopState *st, bool prior) {
+                   F *d2, LoopState *st, bool prior, bool init) {
     return KMB_EUNSUPPORTED;  // float64 data has no tensor-core form
 }
 
 template <>
 int assign_pass_tc<float>(kmb_context *ctx, const float *X, int64_t n, int64_t d, const float *C, int64_t k,
-                          int32_t *labels, float *d2, LoopState *st, bool prior) {
+                          int32_t *labels, float *d2, LoopState *st, bool prior, bool init) {
     kmb::Workspace &ws = ctx->ws;
     cudaStream_t s = ctx->stream;
     kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, &sc->cnorm_max_prev);
+    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, &sc->cnorm_max_prev, init);
     KMB_LAUNCHED();
     kmb::launch_prep_centroids_tc(C, k, d, ws.Chi.ptr, ws.Clo.ptr, (float *)ws.h.ptr, &sc->cnorm_max, st, s);
     int rc;
@@ -344,14 +345,14 @@ int assign_pass_tc<float>(kmb_context *ctx, const float *X, int64_t n, int64_t d
 
 template <typename F>
 int assign_pass(kmb_context *ctx, const F *X, int64_t n, int64_t d, const F *C, int64_t k, bool recheck,
-                int32_t *labels, F *d2, LoopState *st, bool tc = false, bool prior = false) {
+                int32_t *labels, F *d2, LoopState *st, bool tc = false, bool prior = false, bool init = false) {
     ProfRange range("addNTToTaskThreaded");
-    if (tc) return assign_pass_tc<F>(ctx, X, n, d, C, k, labels, d2, st, prior);
+    if (tc) return assign_pass_tc<F>(ctx, X, n, d, C, k, labels, d2, st, prior, init);
     kmb::Workspace &ws = ctx->ws;
     cudaStream_t s = ctx->stream;
     const int64_t kpad = round_up(k, kBN);
     kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, nullptr);
+    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, nullptr, init);
     KMB_LAUNCHED();
     kmb::launch_prep_centroids<F>(C, k, d, kpad, (F *)ws.Ct.ptr, (F *)ws.h.ptr, &sc->cnorm_max, st, s);
     {
@@ -636,10 +637,9 @@ int train_impl(kmb_context *ctx, int memory, const void *Xv, int64_t n, int64_t 
     if ((rc = assign_pass<F>(ctx, X, n, d, Ccur, k, recheck, labels, d2, st_final, tc,
                              /*prior=*/p->max_iteration_count > 0)))
         return rc;
-    double *obj_dev = &sc->objective;
     {
         ProfRange range("kmeansUpdateObjectiveFunction");
-        kmb::launch_objective<F>(X, n, d, Ccur, labels, (double *)ws.obj_part.ptr, obj_dev, s);
+        kmb::launch_objective<F>(X, n, d, Ccur, labels, (double *)ws.obj_part.ptr, &st_final->objective, s);
     }
     KMB_CUDA(cudaGetLastError());
 
@@ -647,15 +647,13 @@ int train_impl(kmb_context *ctx, int memory, const void *Xv, int64_t n, int64_t 
     if (C_out) KMB_CUDA(cudaMemcpyAsync(C_out, Ccur, sizeof(F) * k * d, out_kind, s));
     if (responses && labels != responses)
         KMB_CUDA(cudaMemcpyAsync(responses, labels, sizeof(int32_t) * n, out_kind, s));
-    double obj_h = 0.0;
-    KMB_CUDA(cudaMemcpyAsync(&obj_h, obj_dev, sizeof(double), cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaMemcpyAsync(ctx->h_state, st, sizeof(LoopState) * 2, cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaStreamSynchronize(s));
     const LoopState &hs = ctx->h_state[0];
     if (hs.error) return fail(ctx, hs.error, "device loop failed (status %d)", hs.error);
     if (ctx->h_state[1].error)
         return fail(ctx, ctx->h_state[1].error, "final assignment pass failed (status %d)", ctx->h_state[1].error);
-    if (objective) *objective = obj_h;
+    if (objective) *objective = ctx->h_state[1].objective;
     if (iteration_count) *iteration_count = hs.iterations;
     if (stats) {
         stats->rechecked_rows = ctx->h_state[1].n_recheck + ctx->h_state[1].n_full;
@@ -687,25 +685,20 @@ int infer_impl(kmb_context *ctx, int memory, const void *Xv, int64_t n, int64_t 
     }
     int32_t *labels = (memory == KMB_MEM_DEVICE && responses) ? responses : (int32_t *)ws.labels.ptr;
     LoopState *st = (LoopState *)ws.state.ptr + 1;
-    kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    init_state(ctx->h_state[1], 0.0);
-    KMB_CUDA(cudaMemcpyAsync(st, &ctx->h_state[1], sizeof(LoopState), cudaMemcpyHostToDevice, s));
-    KMB_CUDA(cudaMemsetAsync(sc, 0, sizeof(kmb::DevScalars), s));
     prepare_rows<F>(ctx, X, n, d, tc);
-    if ((rc = assign_pass<F>(ctx, X, n, d, C, k, recheck, labels, (F *)ws.d2.ptr, st, tc))) return rc;
+    if ((rc = assign_pass<F>(ctx, X, n, d, C, k, recheck, labels, (F *)ws.d2.ptr, st, tc, /*prior=*/false, /*init=*/true)))
+        return rc;
     if (compute_objective)
-        kmb::launch_objective<F>(X, n, d, C, labels, (double *)ws.obj_part.ptr, &sc->objective, s);
+        kmb::launch_objective<F>(X, n, d, C, labels, (double *)ws.obj_part.ptr, &st->objective, s);
     KMB_CUDA(cudaGetLastError());
     const cudaMemcpyKind out_kind = memory == KMB_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
     if (responses && labels != responses)
         KMB_CUDA(cudaMemcpyAsync(responses, labels, sizeof(int32_t) * n, out_kind, s));
-    double obj_h = 0.0;
-    KMB_CUDA(cudaMemcpyAsync(&obj_h, &sc->objective, sizeof(double), cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaMemcpyAsync(&ctx->h_state[1], st, sizeof(LoopState), cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaStreamSynchronize(s));
     if (ctx->h_state[1].error)
         return fail(ctx, ctx->h_state[1].error, "assignment pass failed (status %d)", ctx->h_state[1].error);
-    if (compute_objective && objective) *objective = obj_h;
+    if (compute_objective && objective) *objective = ctx->h_state[1].objective;
     if (stats) {
         stats->rechecked_rows = ctx->h_state[1].n_recheck + ctx->h_state[1].n_full;
         stats->full_rescans = ctx->h_state[1].n_full;
@@ -848,12 +841,12 @@ int prepare_csr(kmb_context *ctx, int memory, const void *vals, const int64_t *c
 
 template <typename F>
 void csr_assign_pass(kmb_context *ctx, const kmb::CsrRows &X, const F *C, int64_t k, int32_t *labels, F *d2,
-                     LoopState *st) {
+                     LoopState *st, bool init = false) {
     kmb::Workspace &ws = ctx->ws;
     cudaStream_t s = ctx->stream;
     const int64_t kpad = round_up(k, kBN);
     kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, nullptr);
+    reset_iteration_kernel<<<1, 1, 0, s>>>(st, &sc->cnorm_max, nullptr, init);
     KMB_LAUNCHED();
     kmb::launch_prep_centroids<F>(C, k, X.d, kpad, (F *)ws.Ct.ptr, (F *)ws.h.ptr, &sc->cnorm_max, st, s);
     KernelTimer timer(ctx, 0);
@@ -937,21 +930,19 @@ int train_csr_impl(kmb_context *ctx, int memory, const void *vals, const int64_t
     // responses against the final centroids, then the exact objective
     csr_assign_pass<F>(ctx, X, Ccur, k, labels, d2, st + 1);
     kmb::launch_csr_objective<F>(X, Ccur, k, labels, (double *)ws.csr_cnorm.ptr, (double *)ws.obj_part.ptr,
-                                 &sc->objective, s);
+                                 &st[1].objective, s);
     KMB_CUDA(cudaGetLastError());
     const cudaMemcpyKind out_kind = memory == KMB_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
     if (C_out) KMB_CUDA(cudaMemcpyAsync(C_out, Ccur, sizeof(F) * k * d, out_kind, s));
     if (responses && labels != responses)
         KMB_CUDA(cudaMemcpyAsync(responses, labels, sizeof(int32_t) * n, out_kind, s));
-    double obj_h = 0.0;
-    KMB_CUDA(cudaMemcpyAsync(&obj_h, &sc->objective, sizeof(double), cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaMemcpyAsync(ctx->h_state, st, sizeof(LoopState) * 2, cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaStreamSynchronize(s));
     const LoopState &hs = ctx->h_state[0];
     if (hs.error) return fail(ctx, hs.error, "device loop failed (status %d)", hs.error);
     if (ctx->h_state[1].error)
         return fail(ctx, ctx->h_state[1].error, "final assignment pass failed (status %d)", ctx->h_state[1].error);
-    if (objective) *objective = obj_h;
+    if (objective) *objective = ctx->h_state[1].objective;
     if (iteration_count) *iteration_count = hs.iterations;
     if (stats) {
         std::memset(stats, 0, sizeof(*stats));
@@ -977,22 +968,17 @@ int infer_csr_impl(kmb_context *ctx, int memory, const void *vals, const int64_t
     if (memory == KMB_MEM_HOST && (rc = upload<F>(ctx, ws.C0, Cv, sizeof(F) * k * d, &C))) return rc;
     int32_t *labels = (memory == KMB_MEM_DEVICE && responses) ? responses : (int32_t *)ws.labels.ptr;
     LoopState *st = (LoopState *)ws.state.ptr + 1;
-    kmb::DevScalars *sc = (kmb::DevScalars *)ws.scalars.ptr;
-    init_state(ctx->h_state[1], 0.0);
-    KMB_CUDA(cudaMemcpyAsync(st, &ctx->h_state[1], sizeof(LoopState), cudaMemcpyHostToDevice, s));
-    KMB_CUDA(cudaMemsetAsync(sc, 0, sizeof(kmb::DevScalars), s));
-    csr_assign_pass<F>(ctx, X, C, k, labels, (F *)ws.d2.ptr, st);
+    csr_assign_pass<F>(ctx, X, C, k, labels, (F *)ws.d2.ptr, st, /*init=*/true);
     if (compute_objective)
         kmb::launch_csr_objective<F>(X, C, k, labels, (double *)ws.csr_cnorm.ptr, (double *)ws.obj_part.ptr,
-                                     &sc->objective, s);
+                                     &st->objective, s);
     KMB_CUDA(cudaGetLastError());
     const cudaMemcpyKind out_kind = memory == KMB_MEM_HOST ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
     if (responses && labels != responses)
         KMB_CUDA(cudaMemcpyAsync(responses, labels, sizeof(int32_t) * n, out_kind, s));
-    double obj_h = 0.0;
-    KMB_CUDA(cudaMemcpyAsync(&obj_h, &sc->objective, sizeof(double), cudaMemcpyDeviceToHost, s));
+    KMB_CUDA(cudaMemcpyAsync(&ctx->h_state[1], st, sizeof(LoopState), cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaStreamSynchronize(s));
-    if (compute_objective && objective) *objective = obj_h;
+    if (compute_objective && objective) *objective = ctx->h_state[1].objective;
     return KMB_OK;
 }
 

@@ -174,11 +174,19 @@ __global__ void __launch_bounds__(256) csr_objective_kernel(const F *__restrict_
     }
 }
 
-__global__ void csr_sum_partials_kernel(const double *__restrict__ partials, int count, double *__restrict__ out) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        double s = 0.0;
-        for (int i = 0; i < count; ++i) s += partials[i];
-        *out = s;
+// One block, a fixed order.
+__global__ void __launch_bounds__(256) csr_sum_partials_kernel(const double *__restrict__ partials, int count,
+                                                               double *__restrict__ out) {
+    __shared__ double part[8];
+    double s = 0.0;
+    for (int i = threadIdx.x; i < count; i += 256) s += partials[i];
+    for (int m = 16; m >= 1; m >>= 1) s += __shfl_xor_sync(0xffffffffu, s, m);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int w = 0; w < 8; ++w) t += part[w];
+        *out = t;
     }
 }
 
@@ -222,7 +230,7 @@ void launch_csr_objective(const CsrRows &X, const F *C, int64_t k, const int32_t
     csr_objective_kernel<F><<<kCsrObjectiveBlocks, 256, 0, s>>>((const F *)X.vals, X.cols, X.rowptr, X.n, (int)X.d, C,
                                                                 labels, cnorm2, partials);
     KMB_LAUNCHED();
-    csr_sum_partials_kernel<<<1, 32, 0, s>>>(partials, kCsrObjectiveBlocks, out);
+    csr_sum_partials_kernel<<<1, 256, 0, s>>>(partials, kCsrObjectiveBlocks, out);
     KMB_LAUNCHED();
 }
 
