@@ -53,7 +53,7 @@ namespace batched {
 constexpr int NT = 256;            // threads per CTA
 constexpr int BK = 8;              // contraction chunk of the assignment tile
 constexpr int kMaxK = 256;         // clusters per problem (one assignment tile covers all)
-constexpr int kAccRows = 4096;     // rows per accumulate / setup work item
+constexpr int kAccRows = 4096;     // rows per accumulate / setup work item, at most (Problem::rows)
 constexpr long long kBarrierTimeout = 4000000000ll;  // ~2 s of SM clocks
 
 struct Problem {
@@ -71,6 +71,7 @@ struct Problem {
     int *colexp;        // d (column maxima as float bits during setup, then E_t)
     long long n;
     int d, dpad, k, kpad, tm;
+    int rows;           // rows per work item: a power of two, 512 to kAccRows
     int done, iters, max_iters, empty_events;
     int inc;            // this iteration's accumulation: 0 every row, 1 the moved rows only
     long long moved;    // rows whose label changed in this iteration's work phase
@@ -88,7 +89,7 @@ struct Phase {
 };
 
 struct Lists {
-    Phase blocks;  // (problem, row block of kAccRows): setup
+    Phase blocks;  // (problem, row block): setup
     Phase work;    // its order: every problem, costliest blocks first
     int n_problems;
     int iterations;
@@ -116,7 +117,7 @@ __device__ void compact_active(const Problem *P, const Lists &L, unsigned char *
         if (p.done) continue;
         ++c;
         wp += p.kpad;
-        ww += (p.n + kAccRows - 1) / kAccRows;
+        ww += (p.n + p.rows - 1) / p.rows;
         wf += p.k;
     }
     s_cnt[threadIdx.x] = c;
@@ -157,7 +158,7 @@ __device__ void compact_active(const Problem *P, const Lists &L, unsigned char *
         L.act_fin[o] = af;
         ++o;
         ap += p.kpad;
-        aw += (p.n + kAccRows - 1) / kAccRows;
+        aw += (p.n + p.rows - 1) / p.rows;
         af += p.k;
     }
 }
@@ -167,6 +168,7 @@ struct GridBarrier {
     unsigned gen;
     int error;   // 1: a barrier wait ran out; 2: an invalid label reached the accumulation
     int active;  // problems not yet converged
+    unsigned next;  // work items handed out in this iteration
 };
 
 __device__ __forceinline__ int2 item_of(const Phase &ph, int count, long long i) {
@@ -215,7 +217,7 @@ __device__ void setup_item(Problem &p, int blk, float *smax) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     for (int t = threadIdx.x; t < p.d; t += NT) smax[t] = 0.f;
     __syncthreads();
-    const long long b = (long long)blk * kAccRows, e = min(p.n, b + kAccRows);
+    const long long b = (long long)blk * p.rows, e = min(p.n, b + p.rows);
     for (long long r = b + warp; r < e; r += NT / 32) {
         const float *x = p.X + r * p.d;
         double s = 0.0;
@@ -504,7 +506,7 @@ __device__ __forceinline__ void assign_dispatch(const Problem &p, int pid, int t
 __device__ void accumulate_item(Problem &p, int blk, int *sm, GridBarrier *gb) {
     int *s_cnt = sm, *s_off = sm + kMaxK, *s_fill = sm + 2 * kMaxK, *s_rows = sm + 3 * kMaxK;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long b = (long long)blk * kAccRows, e = min(p.n, b + kAccRows);
+    const long long b = (long long)blk * p.rows, e = min(p.n, b + p.rows);
     const int rows = (int)(e - b);
     const int k = p.k, d = p.d;
     for (int j = threadIdx.x; j < k; j += NT) {
@@ -574,16 +576,28 @@ __device__ void accumulate_item(Problem &p, int blk, int *sm, GridBarrier *gb) {
         const int ec = active ? p.colexp[c] : 0;
         long long a0 = 0, a1 = 0, a2 = 0;
         const int step = S * rps;
-        for (int i = sl * rps + rl; i < cnt; i += 8 * step) {  // eight gathered loads in flight
-            float v[8];
+        Bins bins;
+        if (ec != 0) {
+            const Bins::Magic mg(ec);
+            for (int i = sl * rps + rl; i < cnt; i += 8 * step) {  // eight gathered loads in flight
+                float v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int ii = i + u * step;
-                v[u] = (active && ii < cnt) ? Xb[(long long)s_rows[base + ii] * d + c] : 0.f;
+                for (int u = 0; u < 8; ++u) {
+                    const int ii = i + u * step;
+                    v[u] = ii < cnt ? Xb[(long long)s_rows[base + ii] * d + c] : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) bins.add(v[u], mg);
             }
-#pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const Limbs L = fixed_of(v[u], ec);
+        }
+        if (ec != 0 && bins.finite()) {
+            const Limbs L = bins.limbs(ec);
+            a0 = L.l0;
+            a1 = L.l1;
+            a2 = L.l2;
+        } else if (active) {  // a column of zeros, or non-finite values
+            for (int i = sl * rps + rl; i < cnt; i += step) {
+                const Limbs L = fixed_of(Xb[(long long)s_rows[base + i] * d + c], ec);
                 a0 += L.l0;
                 a1 += L.l1;
                 a2 += L.l2;
@@ -608,7 +622,7 @@ __device__ void accumulate_item(Problem &p, int blk, int *sm, GridBarrier *gb) {
 
 // Full accumulation's bookkeeping: the block's rows that changed label, and prev.
 __device__ void track_item(Problem &p, int blk) {
-    const long long b = (long long)blk * kAccRows, e = min(p.n, b + kAccRows);
+    const long long b = (long long)blk * p.rows, e = min(p.n, b + p.rows);
     int c = 0;
     for (long long r = b + threadIdx.x; r < e; r += NT) {
         const int lab = p.labels[r];
@@ -624,7 +638,7 @@ __device__ void track_item(Problem &p, int blk) {
 // in any order), counts follow, prev follows the labels.
 __device__ void moves_item(Problem &p, int blk, GridBarrier *gb) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long long b = (long long)blk * kAccRows, e = min(p.n, b + kAccRows);
+    const long long b = (long long)blk * p.rows, e = min(p.n, b + p.rows);
     const int k = p.k, d = p.d;
     const long long plane = (long long)k * d;
     unsigned long long *acc = reinterpret_cast<unsigned long long *>(p.acc);
@@ -814,7 +828,10 @@ __global__ void __launch_bounds__(NT, 3) persistent_kernel(Problem *P, Lists L, 
     for (int i = blockIdx.x; i < L.n_problems; i += gridDim.x) scales_item(P[i]);
     if (!grid_sync(gb)) return;
     for (int it = 0; it < L.iterations; ++it) {
-        if (blockIdx.x == 0) compact_active(P, L, smem_raw);
+        if (blockIdx.x == 0) {
+            compact_active(P, L, smem_raw);
+            if (threadIdx.x == 0) gb->next = 0;
+        }
         if (!grid_sync(gb)) return;
         const int na = *(volatile int *)L.act_count;  // the same for every CTA until the next compaction
         const Phase prep{L.act_prep, L.act_order, *(volatile long long *)&L.act_prep[na]};
@@ -826,19 +843,25 @@ __global__ void __launch_bounds__(NT, 3) persistent_kernel(Problem *P, Lists L, 
         }
         if (!grid_sync(gb)) return;
         {
-            // (problem, block of kAccRows rows), round-robin, costliest problems first:
-            // the block's assignment tiles, then its accumulation, which finds the rows
-            // this CTA has just read in L2. A problem with more blocks than the grid has
-            // CTAs gives a CTA consecutive blocks of itself, whose centroids then stay in
-            // shared memory.
+            // (problem, block of its rows), costliest problems first, handed out one
+            // by one: the block's assignment tiles, then its accumulation, which finds the
+            // rows this CTA has just read in L2. Items differ 200-fold in cost; dealt
+            // round-robin, a quarter of the kernel's time was the wait for the CTA with
+            // the largest ones (512 problems, 30 iterations: 96 ms, 77 ms handed out).
             int cached = -1;
             int *acc_smem = reinterpret_cast<int *>(smem_raw + kAssignSmem);
-            for (long long i = blockIdx.x; i < work.items; i += gridDim.x) {
+            for (;;) {
+                __shared__ unsigned s_item;
+                if (threadIdx.x == 0) s_item = atomicAdd(&gb->next, 1u);
+                __syncthreads();
+                const unsigned i = s_item;
+                __syncthreads();  // (read before the next item replaces it)
+                if (i >= work.items) break;
                 const int2 w = item_of(work, na, i);
                 Problem &p = P[w.x];
                 const int bm = rows_per_item(p.tm);
-                const long long t0 = (long long)w.y * (kAccRows / bm);
-                const long long t1 = min((p.n + bm - 1) / bm, t0 + kAccRows / bm);
+                const long long t0 = (long long)w.y * (p.rows / bm);
+                const long long t1 = min((p.n + bm - 1) / bm, t0 + p.rows / bm);
                 for (long long t = t0; t < t1; ++t) assign_dispatch(p, w.x, (int)t, fsm, cached);
                 __syncthreads();  // the block's labels, written by every thread, before they are read
                 if (p.inc) {
@@ -1012,6 +1035,7 @@ void launch_shard_exact_sums(const float *X, int64_t n, int d, int k, const int3
     p.colexp = const_cast<int *>(colexp);
     p.acc = acc;
     p.counts = counts;
+    p.rows = kAccRows;
     const int nblocks = (int)((n + kAccRows - 1) / kAccRows);
     // the accumulation reports an out-of-range label in the error word of a grid barrier
     GridBarrier *gb = reinterpret_cast<GridBarrier *>(reinterpret_cast<char *>(bad) - offsetof(GridBarrier, error));
@@ -1065,6 +1089,14 @@ extern "C" int kmb_batched_train(int dtype, kmb_batched_problem *problems, int64
         arena += (bytes + 255) / 256 * 256;
         return o;
     };
+    // rows per work item: about four items per CTA of the grid (three CTAs per SM) where the
+    // problems are few, so that no CTA's single item outlasts the others' work (8 problems, 19
+    // iterations: 13.5 ms with 4096 rows an item, 3.6 ms with 512; 100 problems 24.7 and
+    // 17.3 ms with 2048)
+    long long total_rows = 0;
+    for (int64_t i = 0; i < count; ++i) total_rows += problems[i].n;
+    int item_rows = 512;
+    while (item_rows < kAccRows && (long long)item_rows * 2 * 12 * sms <= total_rows) item_rows *= 2;
     std::vector<Problem> H(count);
     std::vector<size_t> off((size_t)count * 9);
     for (int64_t i = 0; i < count; ++i) {
@@ -1105,6 +1137,7 @@ extern "C" int kmb_batched_train(int dtype, kmb_batched_problem *problems, int64
         p.dpad = (int)((q.d + 7) / 8 * 8);
         p.k = (int)q.k;
         p.kpad = batched_kpad(p.k);
+        p.rows = item_rows;
         p.tm = tuned_tm(dev, p.dpad, p.kpad, s);
         p.Ct = (float *)(base + off[i * 9 + 0]);
         p.h = (float *)(base + off[i * 9 + 1]);
@@ -1119,14 +1152,14 @@ extern "C" int kmb_batched_train(int dtype, kmb_batched_problem *problems, int64
         p.eps = accuracy_threshold;
         p.done = max_iteration_count == 0 ? 1 : 0;
         classes[(long long)p.kpad * 16 + p.tm] = 1;
-        pre[0 * P1 + i + 1] = pre[0 * P1 + i] + (p.n + kAccRows - 1) / kAccRows;
+        pre[0 * P1 + i + 1] = pre[0 * P1 + i] + (p.n + p.rows - 1) / p.rows;
         pre[1 * P1 + i + 1] = pre[1 * P1 + i] + p.kpad;
         pre[3 * P1 + i + 1] = pre[3 * P1 + i] + p.k;
-        nblocks[i] = (p.n + kAccRows - 1) / kAccRows;
-        block_cost[i] = (double)std::min<long long>(p.n, kAccRows) * p.kpad * p.dpad;
+        nblocks[i] = (p.n + p.rows - 1) / p.rows;
+        block_cost[i] = (double)std::min<long long>(p.n, p.rows) * p.kpad * p.dpad;
         order[i] = (int)i;
     }
-    // work: problems with the costliest blocks first (round-robin over the grid then balances well)
+    // work: problems with the costliest blocks first (handing them out then balances well)
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return block_cost[a] > block_cost[b]; });
     for (int64_t q = 0; q < count; ++q) pre[2 * P1 + q + 1] = pre[2 * P1 + q] + nblocks[order[q]];
     Problem *dP = nullptr;

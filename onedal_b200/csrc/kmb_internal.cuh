@@ -397,7 +397,11 @@ struct Bins {
     struct Magic {
         double a, b, c;
         __device__ __forceinline__ explicit Magic(int e)
-            : a(ldexp(1.5, 52 + 59 - e)), b(ldexp(1.5, 52 + 23 - e)), c(ldexp(1.5, 52 - e)) {}
+            : a(power(52 + 59 - e)), b(power(52 + 23 - e)), c(power(52 - e)) {}
+        // 1.5 * 2^p (|p| < 1000: e lies in [-34, 243])
+        static __device__ __forceinline__ double power(int p) {
+            return __longlong_as_double(((long long)(p + 1023) << 52) | 0x8000000000000ll);
+        }
     };
     __device__ __forceinline__ void add(float x, const Magic &m3) {
         const double v = (double)x;
