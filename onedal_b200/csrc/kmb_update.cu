@@ -767,19 +767,25 @@ __global__ void __launch_bounds__(kTailThreads) update_tail_kernel(const TailArg
 // order. Bound by the row bytes and the float conversions; a thread per column and row took
 // 788 us for 4M x 128 (2.05 GB), 295 us for 3M x 50, 61 us for 1M x 20 and 999 us for 10M x
 // 64: 460, 208, 34 and 553 us here (two or four rows in flight per lane group were slower).
+// Doubles read the next row's label ahead of a row's values (3M x 33: 300 -> 236 us, 9.6M x 64:
+// 1311 -> 1157 us); floats do not (9M x 64: 503 us, with it 667 us).
 template <typename F, int W, int L>
 __global__ void __launch_bounds__(256)
 objective_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restrict__ C, const int32_t *__restrict__ labels,
                  double *__restrict__ partials) {
     constexpr int RP = 32 / L;  // rows a warp reads side by side
+    constexpr bool kAhead = sizeof(F) == 8;
     __shared__ double part[8];
     struct alignas(sizeof(F) * W) Vec { F v[W]; };
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, sub = lane % L, group = lane / L;
     const int64_t per = (n + gridDim.x - 1) / gridDim.x;
     const int64_t b = (int64_t)blockIdx.x * per, e = min(n, b + per);
     double acc = 0.0;
-    for (int64_t r = b + (int64_t)warp * RP + group; r < e; r += 8 * RP) {
-        const F *x = X + r * d, *c = C + (int64_t)labels[r] * d;
+    int64_t r = b + (int64_t)warp * RP + group;
+    int32_t next = kAhead && r < e ? labels[r] : 0;
+    for (; r < e; r += 8 * RP) {
+        const F *x = X + r * d, *c = C + (int64_t)(kAhead ? next : labels[r]) * d;
+        if (kAhead && r + 8 * RP < e) next = labels[r + 8 * RP];
         for (int t = sub * W; t < d; t += L * W) {
             const Vec xv = *reinterpret_cast<const Vec *>(x + t), cv = *reinterpret_cast<const Vec *>(c + t);
             double xd[W], cd[W];
