@@ -566,6 +566,12 @@ constexpr int kSmallThreads = 128;
 // cluster accumulates x_t * c_t in ascending t, as the other kernels do, so the
 // scores -- and the labels, distances and recheck entries -- are the same; only
 // the 128-cluster tile padding and the tile epilogue are gone.
+// d > 32: bound by the rows' bytes, and a thread that reads its own row straight from memory
+// touches 32 lines a load (9M x 64 floats 2436 us, 0.95 TB/s; 9.6M x 64 doubles 2948 us). Each
+// warp copies its 32 rows side by side into an odd-strided tile, moves them to registers and
+// has the next rows on their way while it works, four clusters at a time since one dot
+// product is a chain of d FMAs: 841 and 1608 us. Shorter rows stay in L1 between a thread's
+// loads and are read directly (5M x 17, k = 31 floats: 410 us, through the tile 501 us).
 template <typename F, int DMAX>
 __global__ void __launch_bounds__(kSmallThreads)
 assign_small_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restrict__ Ct, const F *__restrict__ h,
@@ -575,6 +581,9 @@ assign_small_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restri
     if (st && st->done) return;
     __shared__ __align__(16) F Cs[kSmallK][DMAX];
     __shared__ F hs[kSmallK];
+    extern __shared__ __align__(16) unsigned char small_rows[];
+    constexpr bool kTile = DMAX > 32;
+    constexpr int QN = kTile ? 4 : 1;  // clusters at a time
     for (int i = threadIdx.x; i < kSmallK * DMAX; i += blockDim.x) {
         const int j = i / DMAX, t = i % DMAX;
         Cs[j][t] = (j < k && t < d) ? Ct[(int64_t)t * kpad + j] : F(0);
@@ -583,25 +592,61 @@ assign_small_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restri
     __syncthreads();
     const double u = unit_roundoff<F>();
     const double cmax = cnorm_max ? *cnorm_max : 0.0;
-    for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31, ld = d | 1;
+    F *tile = reinterpret_cast<F *>(small_rows) + (threadIdx.x >> 5) * 32 * ld;
+    const int64_t step = (int64_t)gridDim.x * kSmallThreads;
+    auto copy_rows = [&](int64_t first) {  // rows [first, first + 32) below n: one run of memory
+        const int total = first < n ? (int)min((int64_t)32, n - first) * d : 0;
+        const F *src = X + first * d;
+        for (int i = lane, r = 0, t = lane; i < total; i += 32, t += 32) {
+            if (t >= d) {  // d > 32: one row on at most
+                t -= d;
+                ++r;
+            }
+            cp_async_zfill(&tile[r * ld + t], src + i, (int)sizeof(F), true);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // The warp's first row, or the thread's own where it reads directly.
+    int64_t first = (int64_t)blockIdx.x * kSmallThreads + (kTile ? threadIdx.x & ~31 : threadIdx.x);
+    if (kTile) copy_rows(first);
+    for (; first < n; first += step) {
+        const int64_t r = first + (kTile ? lane : 0);
         F x[DMAX];
-        const F *xr = X + r * (int64_t)d;
+        if constexpr (kTile) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncwarp();
 #pragma unroll
-        for (int t = 0; t < DMAX; ++t) x[t] = t < d ? xr[t] : F(0);
+            for (int t = 0; t < DMAX; ++t) x[t] = t < d ? tile[lane * ld + t] : F(0);
+            __syncwarp();
+            copy_rows(first + step);
+            if (r >= n) continue;
+        } else {
+            const F *xr = X + r * (int64_t)d;
+#pragma unroll
+            for (int t = 0; t < DMAX; ++t) x[t] = t < d ? xr[t] : F(0);
+        }
         RowTop<F> top;
         top.b = top.s = top.t = f_inf<F>();
         top.ib = top.is = 0;
-        for (int j = 0; j < k; ++j) {
-            F dot = F(0);
+        for (int j = 0; j < k; j += QN) {
+            F dot[QN];
+#pragma unroll
+            for (int q = 0; q < QN; ++q) dot[q] = F(0);
 #pragma unroll
             for (int t = 0; t < DMAX; t += 4) {
-                const typename Vec4<F>::T c = *reinterpret_cast<const typename Vec4<F>::T *>(&Cs[j][t]);
-                dot = fma(x[t], c.x, dot);
-                dot = fma(x[t + 1], c.y, dot);
-                dot = fma(x[t + 2], c.z, dot);
-                dot = fma(x[t + 3], c.w, dot);
+#pragma unroll
+                for (int q = 0; q < QN; ++q) {
+                    const typename Vec4<F>::T c = *reinterpret_cast<const typename Vec4<F>::T *>(&Cs[j + q][t]);
+                    dot[q] = fma(x[t], c.x, dot[q]);
+                    dot[q] = fma(x[t + 1], c.y, dot[q]);
+                    dot[q] = fma(x[t + 2], c.z, dot[q]);
+                    dot[q] = fma(x[t + 3], c.w, dot[q]);
+                }
             }
-            top_push(top, hs[j] - dot, j);
+#pragma unroll
+            for (int q = 0; q < QN; ++q)
+                if (j + q < k) top_push(top, hs[j + q] - dot[q], j + q);
         }
         labels[r] = top.ib;
         const F xn = xnorm[r];
@@ -614,6 +659,7 @@ assign_small_kernel(const F *__restrict__ X, int64_t n, int d, const F *__restri
                 enqueue_recheck(queue, n, st, (int)r, top.ib, top.is, (double)top.t - (double)top.b <= band);
         }
     }
+    if (kTile) asm volatile("cp.async.wait_group 0;" ::: "memory");
 }
 
 // ---- FP32, centroids resident in shared memory ------------------------------
@@ -1045,8 +1091,14 @@ void launch_small(const F *X, int64_t n, int64_t d, const F *Ct, const F *h, int
                   const double *cnorm_max, int32_t *labels, F *d2, RecheckEntry *queue, LoopState *st,
                   cudaStream_t s) {
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((n + kSmallThreads - 1) / kSmallThreads, 148 * 16));
-    assign_small_kernel<F, DMAX><<<(unsigned)blocks, kSmallThreads, 0, s>>>(X, n, (int)d, Ct, h, (int)k, (int)kpad,
-                                                                           xnorm, cnorm_max, labels, d2, queue, st);
+    size_t smem = 0;
+    if (DMAX > 32) {  // the tiles; the limit is the largest d's in every call, as threads set it side by side
+        smem = sizeof(F) * kSmallThreads * (d | 1);
+        cudaFuncSetAttribute(assign_small_kernel<F, DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)(sizeof(F) * kSmallThreads * (DMAX | 1)));
+    }
+    assign_small_kernel<F, DMAX><<<(unsigned)blocks, kSmallThreads, smem, s>>>(X, n, (int)d, Ct, h, (int)k, (int)kpad,
+                                                                              xnorm, cnorm_max, labels, d2, queue, st);
     KMB_LAUNCHED();
 }
 
