@@ -136,6 +136,17 @@ cudaMemPool_t library_pool(int dev) {
     return pool;
 }
 
+cudaError_t allow_smem(const void *kern) {
+    int dev = 0, optin = 0;
+    cudaFuncAttributes a;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&a, kern);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)a.sharedSizeBytes);
+    return e;
+}
+
 std::mutex &cooperative_mutex() {
     static std::mutex mu;
     return mu;
@@ -1266,6 +1277,7 @@ int init_plusplus_core(kmb_context *ctx, int memory, const F *X, const kmb::CsrR
         else
             kmb::launch_pp_rounds<F>(X, n, d, k, c_begin, update_first, md, acc, (unsigned *)ws.pp_flags.ptr, rnd,
                                      rnd + k, pool_n, C, st, s);
+        KMB_CUDA(cudaGetLastError());  // (a refused launch would leave distances of earlier rounds)
         KMB_CUDA(cudaMemcpyAsync(&hs, st, sizeof(hs), cudaMemcpyDeviceToHost, s));
         KMB_CUDA(cudaStreamSynchronize(s));
         if (!hs.stopped) break;

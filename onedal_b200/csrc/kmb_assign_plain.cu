@@ -1176,7 +1176,7 @@ bool launch_resident<float>(const float *X, int64_t n, int64_t d, const float *C
                                     assign_resident_kernel<128, 1, true, T3>, assign_resident_kernel<0, 1, true, T3>);
     };
     auto kern = queue ? pick(std::true_type()) : pick(std::false_type());
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    if (allow_smem((const void *)kern) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }

@@ -1490,7 +1490,7 @@ int launch_assign_tc(const void *Xhi, const void *Xlo, int64_t n, int64_t d, con
     if (own) {
         auto kern = products == 1 ? (bn == 256 ? tc::assign_tc_own_kernel<256, 1> : tc::assign_tc_own_kernel<128, 1>)
                                   : (bn == 256 ? tc::assign_tc_own_kernel<256, 3> : tc::assign_tc_own_kernel<128, 3>);
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (allow_smem((const void *)kern) != cudaSuccess)
             return KMB_ECUDA;
         const int grid = num_sms < 0 ? p.n_tiles : (int)std::min<int64_t>(num_sms, p.n_tiles);
         kern<<<grid, tc::NTHREADS, smem, s>>>(mXh, mXl, mCh, mCl, p);
@@ -1500,7 +1500,7 @@ int launch_assign_tc(const void *Xhi, const void *Xlo, int64_t n, int64_t d, con
     if (!pair) {
         auto kern = products == 1 ? (bn == 256 ? tc::assign_tc_kernel<256, false, 1> : tc::assign_tc_kernel<128, false, 1>)
                                   : (bn == 256 ? tc::assign_tc_kernel<256, false, 3> : tc::assign_tc_kernel<128, false, 3>);
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        if (allow_smem((const void *)kern) != cudaSuccess)
             return KMB_ECUDA;
         // num_sms < 0: one CTA per 128-row tile (no persistence), so that other
         // streams' launches interleave with this one at tile granularity
@@ -1512,7 +1512,7 @@ int launch_assign_tc(const void *Xhi, const void *Xlo, int64_t n, int64_t d, con
     // CTA pairs: clusters of two CTAs, one 256-row unit per cluster at a time.
     auto kern = products == 1 ? (bn == 256 ? tc::assign_tc_kernel<256, true, 1> : tc::assign_tc_kernel<128, true, 1>)
                               : (bn == 256 ? tc::assign_tc_kernel<256, true, 3> : tc::assign_tc_kernel<128, true, 3>);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+    if (allow_smem((const void *)kern) != cudaSuccess)
         return KMB_ECUDA;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];

@@ -974,7 +974,7 @@ int tuned_tm(int dev, int dpad, int kpad, cudaStream_t s) {
         tune_fill_kernel<<<64, 256, 0, s>>>(xn, n, 4u);
         launch_count() += 4;
         const size_t smem = smem_bytes(kpad, 1);
-        cudaFuncSetAttribute(tune_assign_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        allow_smem((const void *)tune_assign_kernel);
         float best_ms = 1e30f;
         for (int tm : cands) {
             Problem p;
@@ -1198,7 +1198,7 @@ extern "C" int kmb_batched_train(int dtype, kmb_batched_problem *problems, int64
     const size_t smem = smem_bytes(kmax, dmax);
     int per_sm = 0;
     if (rc == KMB_OK &&
-        (cudaFuncSetAttribute(persistent_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        (allow_smem((const void *)persistent_kernel) != cudaSuccess ||
          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, persistent_kernel, NT, smem) != cudaSuccess ||
          per_sm < 1))
         rc = KMB_EUNSUPPORTED;

@@ -738,7 +738,7 @@ void launch_pp_rounds(const F *X, int64_t n, int64_t d, int64_t k, int64_t c_beg
     const int w = (d * sizeof(F)) % 16 == 0 ? 16 / (int)sizeof(F) : d % 2 == 0 && sizeof(F) == 4 ? 2 : 1;
     auto rows_kernel = w == 1 ? pp_update_rows_kernel<F, 1> : w == 2 ? pp_update_rows_kernel<F, 2> : pp_update_rows_kernel<F, 16 / (int)sizeof(F)>;
     const bool rows = !async && ((uintptr_t)X % 16) == 0 && d <= (1 << 12) && rows_smem <= kRowsMaxSmem &&
-                      cudaFuncSetAttribute(rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, rows_smem) == cudaSuccess;
+                      allow_smem((const void *)rows_kernel) == cudaSuccess;
     for (int64_t c = c_begin; c < k; ++c) {
         if (c > c_begin || update_first) {
             if (rows)

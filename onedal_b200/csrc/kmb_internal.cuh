@@ -85,6 +85,11 @@ __device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived) {
     return s_grid_ok != 0;
 }
 
+// Lets `kern` take all the shared memory of a CTA beside its static part. The limit is one
+// per kernel and device, shared by every host thread: were it each call's own size, a thread
+// with less would refuse the launches of another that needs more.
+cudaError_t allow_smem(const void *kern);
+
 // Recheck queue entry written by the assignment kernels for near-tie rows.
 struct RecheckEntry {
     int row;

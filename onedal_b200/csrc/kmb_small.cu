@@ -725,7 +725,7 @@ cudaError_t launch_small_train(const SmallPlan &p, const F *X, int64_t n, int64_
     if (e != cudaSuccess) return e;
     const size_t smem = small_layout<F>(p.rows, (int)d, (int)k, dmax).total;
     const void *kern = kernel_of<F>(dmax);
-    if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return e;
+    if ((e = allow_smem(kern)) != cudaSuccess) return e;
     void *args[] = {&a};
     e = cudaLaunchCooperativeKernel(kern, dim3((unsigned)p.ctas), dim3(kNT), args, smem, s);
     if (e == cudaSuccess) KMB_LAUNCHED();

@@ -1657,7 +1657,7 @@ void prepare_exact_update_csr(const CsrRows &X, Workspace &ws, LoopState *st, cu
     cudaMemsetAsync(colexp, 0, sizeof(int) * d, s);
     const bool in_smem = (size_t)d * sizeof(unsigned) <= (size_t)96 * 1024;
     const size_t smem = in_smem ? sizeof(unsigned) * d : 0;
-    if (in_smem) cudaFuncSetAttribute(csr_colmax_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (in_smem) allow_smem((const void *)csr_colmax_kernel);
     const unsigned blocks =
         (unsigned)std::max<int64_t>(1, std::min<int64_t>((X.nnz + 255) / 256, in_smem ? 148 * 2 : 148 * 8));
     csr_colmax_kernel<<<blocks, 256, smem, s>>>((const float *)X.vals, X.cols, X.nnz, d, in_smem, (unsigned *)colexp);
