@@ -136,6 +136,12 @@ cudaMemPool_t library_pool(int dev) {
     return pool;
 }
 
+long long grid_wait_cycles() {
+    const char *e = getenv("KMB_GRID_WAIT_LIMIT_CYCLES");
+    const long long v = e ? atoll(e) : 0;
+    return v > 0 && v < kGridTimeout ? v : kGridTimeout;
+}
+
 cudaError_t allow_smem(const void *kern) {
     int dev = 0, optin = 0;
     cudaFuncAttributes a;
@@ -1152,8 +1158,10 @@ int train_spmd_impl(kmb_context *ctx, int dtype, const F *X, int64_t n, int64_t 
             // every rank offers its m farthest rows; the global m farthest by (distance
             // descending, global row ascending) reseed the empty clusters, ascending
             const int m = (int)hids.size(), take = (int)std::min<int64_t>(m, n);
-            if (!kmb::launch_top_rows<F>(row_sq, n, take, ws, (LoopState *)ws.sp_state.ptr, rows, s))
-                return fail(ctx, KMB_ENOMEM, "candidate selection buffers");
+            LoopState *sel_st = (LoopState *)ws.sp_state.ptr, hsel;
+            if ((rc = kmb::launch_top_rows<F>(row_sq, n, take, ws, sel_st, rows, s)))
+                return fail(ctx, rc, "candidate selection not launched (status %d)", rc);
+            KMB_CUDA(cudaMemcpyAsync(&hsel, sel_st, sizeof(hsel), cudaMemcpyDeviceToHost, s));
             if (take > 0) {
                 spmd_gather_kernel<F><<<(unsigned)std::min(take, 1024), 128, 0, s>>>(X, (int)d, rows, row_sq, take,
                                                                                       gvals, gvecs);
@@ -1171,7 +1179,9 @@ int train_spmd_impl(kmb_context *ctx, int dtype, const F *X, int64_t n, int64_t 
                 KMB_CUDA(cudaMemcpyAsync(hvecs.data(), gvecs, sizeof(F) * take * d, cudaMemcpyDeviceToHost, s));
             }
             KMB_CUDA(cudaMemcpyAsync(hC.data(), Ccur, sizeof(F) * kd, cudaMemcpyDeviceToHost, s));
+            KMB_CUDA(cudaGetLastError());
             KMB_CUDA(cudaStreamSynchronize(s));
+            if (hsel.error) return fail(ctx, hsel.error, "candidate selection failed (status %d)", hsel.error);
             for (int e = 0; e < m; ++e) {
                 unsigned char *r = send.data() + rec * e;
                 const double v = e < take ? (std::isnan(hvals[e]) ? -INFINITY : hvals[e]) : -INFINITY;

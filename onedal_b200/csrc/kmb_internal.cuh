@@ -52,14 +52,18 @@ struct GridSync {
 };
 
 constexpr long long kGridTimeout = 4000000000ll;  // ~2 s of SM clocks per wait
+// The limit of a launch's waits: kGridTimeout, or less by KMB_GRID_WAIT_LIMIT_CYCLES in the
+// environment (tests make a wait run out).
+long long grid_wait_cycles();
 
 // Every CTA of the grid arrives before any leaves (cooperative launch: all CTAs are
 // resident); `arrived` counts this CTA's barriers, from zero. One release-add and acquire
 // polls of a count that only grows: about 1500 cycles, where a barrier with a generation
-// word, a reset and full fences took 5000. The wait is bounded; false when this CTA's ran
-// out, which is recorded in sy->error (the others' then run out too). Thread 0 decides
-// and the CTA follows, so all its threads take the same path.
-__device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived) {
+// word, a reset and full fences took 5000. The wait is bounded by `limit` cycles; false when
+// this CTA's ran out, which is recorded in sy->error (the others' then run out too; the
+// caller reports it). Thread 0 decides and the CTA follows, so all its threads take the same
+// path.
+__device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived, long long limit) {
     __shared__ int s_grid_ok;
     __syncthreads();
     ++arrived;
@@ -73,7 +77,7 @@ __device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived) {
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&sy->count) : "memory");
             if (seen >= target) break;
-            if (clock64() - t0 > kGridTimeout) {
+            if (clock64() - t0 > limit) {
                 atomicExch(&sy->error, 1);
                 ok = 0;
                 break;
@@ -478,10 +482,11 @@ void launch_update_exact(const float *X, const UpdatePlan &p, int32_t *labels, c
                          float *C_new, Workspace &ws, LoopState *st, bool commit, cudaStream_t s, float *exact_d2);
 
 // The m rows with the largest d2, in (d2 descending, row ascending) order, into
-// rows_out (device, m int64); m <= n. st is scratch device state (its n_empty is set
-// to m). The sharded training's reseed candidates. False when a buffer cannot grow.
+// rows_out (device, m int64); 0 <= m <= n. The sharded training's reseed candidates. st:
+// device state, cleared here; its error is set when a grid barrier's wait ran out (rows_out
+// then holds rows in range, but not the answer). A status when nothing was launched.
 template <typename F>
-bool launch_top_rows(const F *d2, int64_t n, int m, Workspace &ws, LoopState *st, long long *rows_out, cudaStream_t s);
+int launch_top_rows(const F *d2, int64_t n, int m, Workspace &ws, LoopState *st, long long *rows_out, cudaStream_t s);
 
 // Sharded float training with exact sums (kmb_train_spmd): the column maxima of a
 // shard as float bits (|x| of non-NaN values; 0 for an all-zero column), the

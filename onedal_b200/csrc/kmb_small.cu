@@ -92,6 +92,7 @@ struct SmallArgs {
     SmallCand *cand;   // [CTA][k]
     long long *sel;    // k
     double *obj_part;  // CTA
+    long long wait;    // cycles, of every barrier
 };
 
 // Segments of the accumulation's row list: a thread per (segment, column).
@@ -375,7 +376,7 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
             for (int o = 16; o >= 1; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
             if (lane == 0 && m > 0.f) atomicMax(&a.colbits[t], __float_as_uint(m));
         }
-        ok = grid_sync(sync, arrived);
+        ok = grid_sync(sync, arrived, a.wait);
         for (int t = tid; t < d; t += kNT) {
             const unsigned bits = __ldcg(a.colbits + t);
             const float m = __uint_as_float(bits);
@@ -474,7 +475,7 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
                 a.part[((size_t)l * cells + cell) * G + b] = *reinterpret_cast<unsigned long long *>(&s.v[l]);
         }
         for (int j = tid; j < k; j += kNT) a.part_cnt[(size_t)j * G + b] = start[j + 1] - start[j];
-        if (!(ok = grid_sync(sync, arrived))) break;
+        if (!(ok = grid_sync(sync, arrived, a.wait))) break;
         // finalize: one warp per cell over the grid
         for (int cell = b * kNW + warp; cell < cells; cell += G * kNW) {
             const int j = cell / d, t = cell - j * d;
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
                 if (t == 0) a.counts[j] = cnt;
             }
         }
-        if (!(ok = grid_sync(sync, arrived))) break;
+        if (!(ok = grid_sync(sync, arrived, a.wait))) break;
         // every CTA: the new centroids, the shift, the empty clusters
         double part = 0.0;
         for (int i = tid; i < cells; i += kNT) {
@@ -536,7 +537,7 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
                 }
                 if (rank < have) mine[rank] = SmallCand{key, (long long)(row0 + r)};
             }
-            if (!(ok = grid_sync(sync, arrived))) break;
+            if (!(ok = grid_sync(sync, arrived, a.wait))) break;
             for (int e = warp; e < have; e += kNW) {
                 const unsigned long long key = __ldcg(&mine[e].key);
                 const long long row = __ldcg(&mine[e].row);
@@ -558,7 +559,7 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
                 before = __reduce_add_sync(0xffffffffu, before);
                 if (lane == 0 && before < ne) a.sel[before] = row;
             }
-            if (!(ok = grid_sync(sync, arrived))) break;
+            if (!(ok = grid_sync(sync, arrived, a.wait))) break;
             if (warp == 0) {  // the empty clusters' ids, ascending, in seg
                 int base = 0;
                 for (int j0 = 0; j0 < k; j0 += 32) {
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
         }
         s = cta_sum(s, s_red);
         if (tid == 0) a.obj_part[b] = s;
-        ok = grid_sync(sync, arrived);
+        ok = grid_sync(sync, arrived, a.wait);
         if (ok && b == 0) {
             double v = 0.0;
             for (int c = tid; c < G; c += kNT) v += __ldcg(a.obj_part + c);
@@ -721,6 +722,7 @@ cudaError_t launch_small_train(const SmallPlan &p, const F *X, int64_t n, int64_
     a.cand = (SmallCand *)take(sizeof(SmallCand) * k * G);
     a.sel = (long long *)take(sizeof(long long) * k);
     a.obj_part = (double *)take(sizeof(double) * G);
+    a.wait = grid_wait_cycles();
     cudaError_t e = cudaMemsetAsync(scratch, 0, small_head(d), s);
     if (e != cudaSuccess) return e;
     const size_t smem = small_layout<F>(p.rows, (int)d, (int)k, dmax).total;

@@ -442,7 +442,7 @@ __device__ void cand_sort(Cand *buf, int P) {
 // 1.8 ms at 10M; with the grid collecting, ten updates that each reseed take 3.5 ms less
 // at 1M x 20, k = 1000 (whole train 11.0 -> 7.5 ms) and 22 ms less at 10M x 64, k = 256.
 template <typename F>
-__device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, unsigned &arrived,
+__device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, unsigned &arrived, long long wait,
                            Cand *__restrict__ cand) {
     using K = KeyOf<F>;
     __shared__ unsigned s_hist[kSelBins];
@@ -477,7 +477,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
         __syncthreads();
         for (int i = tid; i < kSelBins; i += kTailThreads)
             if (s_hist[i]) atomicAdd(&sy->hist[round][i], s_hist[i]);
-        if (!grid_sync(sy, arrived)) return false;
+        if (!grid_sync(sy, arrived, wait)) return false;
         // the digit that holds the need-th largest: bins in descending order, four a thread
         unsigned c[4], sum = 0;
 #pragma unroll
@@ -531,7 +531,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
             }
         }
     }
-    if (!grid_sync(sy, arrived)) return false;
+    if (!grid_sync(sy, arrived, wait)) return false;
     if (blockIdx.x == 0) {
         if (!all_eq) {
             if (tid == 0) s_base = (unsigned)m - need;
@@ -576,7 +576,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
             cand_sort(cand, P);
         }
     }
-    return grid_sync(sy, arrived);
+    return grid_sync(sy, arrived, wait);
 }
 
 // Exact squared distances for the empty-cluster candidates: when some cluster is
@@ -602,12 +602,17 @@ __global__ void refresh_d2_kernel(const F *__restrict__ X, int64_t n, int d, con
     }
 }
 
-// The m rows with the largest d2, in (d2 descending, row ascending) order.
+// The m rows with the largest d2, in (d2 descending, row ascending) order. A wait that runs
+// out is recorded in st->error, and rows may keep what they held.
 template <typename F>
 __global__ void __launch_bounds__(kTailThreads)
-top_rows_kernel(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, Cand *cand, long long *__restrict__ rows) {
+top_rows_kernel(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, long long wait, Cand *cand,
+                long long *__restrict__ rows, LoopState *st) {
     unsigned arrived = 0;
-    if (!select_top<F>(d2, n, m, sy, arrived, cand)) return;
+    if (!select_top<F>(d2, n, m, sy, arrived, wait, cand)) {
+        if (threadIdx.x == 0) st->error = KMB_ETIMEDOUT;
+        return;
+    }
     if (blockIdx.x == 0)
         for (int e = threadIdx.x; e < m; e += kTailThreads) rows[e] = __ldcg(&cand[e].row);
 }
@@ -632,6 +637,7 @@ struct TailArgs {
     TailSync *sy;
     LoopState *st;
     int commit;
+    long long wait;  // cycles, of every barrier
 };
 
 // The end of an update, one cooperative launch after the finalize kernel: the
@@ -684,8 +690,8 @@ __global__ void __launch_bounds__(kTailThreads) update_tail_kernel(const TailArg
             }
         }
         unsigned arrived = 0;
-        ok = grid_sync(a.sy, arrived);
-        if (ok) ok = select_top<F>(a.d2, a.n, ne, a.sy, arrived, a.cand);
+        ok = grid_sync(a.sy, arrived, a.wait);
+        if (ok) ok = select_top<F>(a.d2, a.n, ne, a.sy, arrived, a.wait, a.cand);
         if (!ok) {
             if (tid == 0) {
                 st->error = KMB_ETIMEDOUT;
@@ -721,7 +727,7 @@ __global__ void __launch_bounds__(kTailThreads) update_tail_kernel(const TailArg
             }
             __syncthreads();
         }
-        if (a.commit && !grid_sync(a.sy, arrived)) {
+        if (a.commit && !grid_sync(a.sy, arrived, a.wait)) {
             if (tid == 0) {
                 st->error = KMB_ETIMEDOUT;
                 st->done = 1;
@@ -1539,6 +1545,7 @@ static void launch_tail(const F *X, const UpdatePlan &p, const int32_t *labels, 
     a.sy = (TailSync *)ws.sel_state.ptr;
     a.st = st;
     a.commit = commit ? 1 : 0;
+    a.wait = grid_wait_cycles();
     void *args[] = {&a};
     cudaLaunchCooperativeKernel((const void *)update_tail_kernel<F>, dim3((unsigned)tail_grid(p.n, p.k * p.d)),
                                 dim3(kTailThreads), args, 0, s);
@@ -1601,23 +1608,28 @@ void prepare_exact_update(const float *X, int64_t n, int64_t d, Workspace &ws, L
 }
 
 template <typename F>
-bool launch_top_rows(const F *d2, int64_t n, int m, Workspace &ws, LoopState *st, long long *rows_out, cudaStream_t s) {
-    if (m <= 0 || m > n) return m == 0;
+int launch_top_rows(const F *d2, int64_t n, int m, Workspace &ws, LoopState *st, long long *rows_out, cudaStream_t s) {
+    if (m < 0 || m > n) return KMB_EINVAL;
+    cudaMemsetAsync(st, 0, sizeof(LoopState), s);
+    if (m == 0) return KMB_OK;
     int64_t pm = 1;
     while (pm < m) pm <<= 1;
-    if (!ws.ensure(ws.sel_state, sizeof(TailSync)) || !ws.ensure(ws.cand, sizeof(Cand) * pm))
-        return false;
+    if (!ws.ensure(ws.sel_state, sizeof(TailSync)) || !ws.ensure(ws.cand, sizeof(Cand) * pm)) return KMB_ENOMEM;
     TailSync *sy = (TailSync *)ws.sel_state.ptr;
     Cand *cand = (Cand *)ws.cand.ptr;
+    long long wait = grid_wait_cycles();
     cudaMemsetAsync(sy, 0, sizeof(TailSync), s);
-    void *args[] = {(void *)&d2, (void *)&n, (void *)&m, (void *)&sy, (void *)&cand, (void *)&rows_out};
-    cudaLaunchCooperativeKernel((const void *)top_rows_kernel<F>, dim3((unsigned)tail_grid(n, 0)), dim3(kTailThreads),
-                                args, 0, s);
+    cudaMemsetAsync(rows_out, 0, sizeof(long long) * m, s);
+    void *args[] = {(void *)&d2, (void *)&n, (void *)&m, (void *)&sy, (void *)&wait, (void *)&cand, (void *)&rows_out,
+                    (void *)&st};
+    if (cudaLaunchCooperativeKernel((const void *)top_rows_kernel<F>, dim3((unsigned)tail_grid(n, 0)),
+                                    dim3(kTailThreads), args, 0, s) != cudaSuccess)
+        return KMB_ECUDA;
     KMB_LAUNCHED();
-    return true;
+    return KMB_OK;
 }
-template bool launch_top_rows<float>(const float *, int64_t, int, Workspace &, LoopState *, long long *, cudaStream_t);
-template bool launch_top_rows<double>(const double *, int64_t, int, Workspace &, LoopState *, long long *, cudaStream_t);
+template int launch_top_rows<float>(const float *, int64_t, int, Workspace &, LoopState *, long long *, cudaStream_t);
+template int launch_top_rows<double>(const double *, int64_t, int, Workspace &, LoopState *, long long *, cudaStream_t);
 
 void launch_update_exact(const float *X, const UpdatePlan &p, int32_t *labels, const float *d2, float *C_old,
                          float *C_new, Workspace &ws, LoopState *st, bool commit, cudaStream_t s, float *exact_d2) {

@@ -4,6 +4,9 @@
   get a short limit (KMB_TC_WAIT_LIMIT_CYCLES, read at launch); the launch must
   drain its own copies and MMAs, report KMB_ETIMEDOUT, and leave the context
   usable for a correct call afterwards.
+* A grid barrier's wait that runs out (KMB_GRID_WAIT_LIMIT_CYCLES, read at launch): the
+  small train, the update's last launch and the sharded train's candidate selection
+  report KMB_ETIMEDOUT, and the context trains correctly afterwards.
 * Host-side allocation failure (KMB_FAIL_ALLOC=1 makes every workspace growth
   fail): KMB_ENOMEM, raised as bad_alloc by the Python mirror and as oneDAL's
   host_bad_alloc by the dispatcher (backend/interop/error_converter.cpp maps
@@ -13,6 +16,7 @@
   kmeans_lloyd_postprocessing.h:95-130), so a row whose scores are all NaN gets
   cluster 0; the other rows are unaffected.
 """
+import ctypes
 import os
 import subprocess
 
@@ -50,6 +54,57 @@ def test_tensor_core_wait_limit_reports_timeout_and_context_recovers(form, monke
     np.testing.assert_array_equal(r.get_responses().ravel(), lab64)
     t = kmeans.train(desc.set_max_iteration_count(3), X, C)
     assert t.get_iteration_count() == 3
+
+
+def _train(dt, n, k, T):
+    rng = np.random.default_rng(n)
+    X = torch.from_numpy(rng.standard_normal((n, 20)).astype(dt)).cuda()
+    C = X[:k].clone()
+    C[-3:] = 1e4  # nobody's nearest
+    desc = kmeans.descriptor(dt).set_cluster_count(k).set_max_iteration_count(T)
+    desc.set_compute_form(kmeans.compute_form.plain)
+
+    def run():
+        r = kmeans.train(desc, X, C)
+        return r.get_model().get_centroids(), r.get_responses()
+    return run
+
+
+def _train_sharded(dt, n, k, T):
+    rng = np.random.default_rng(n)
+    X = torch.from_numpy(rng.standard_normal((n, 20)).astype(dt)).cuda()
+    C0 = X[:k].clone()
+    C0[-3:] = 1e4
+    gather = _native.ALLGATHER_FN(lambda _u, send, nbytes, recv: ctypes.memmove(recv, send, nbytes) and 0)
+    comm = _native.kmb_communicator(None, 0, 1, _native.ALLREDUCE_F64_FN(lambda _u, _b, _c: 0), gather)
+    p = _native.kmb_params(k, T, 0.0, _native.KMB_FORM_PLAIN, 0)
+
+    def run():
+        ctx = _native.context(0)
+        ctx.set_stream(torch.cuda.current_stream().cuda_stream)
+        C, lab = torch.empty_like(C0), torch.empty(n, dtype=torch.int32, device="cuda")
+        obj, it = ctypes.c_double(), ctypes.c_int64()
+        ctx.check(ctx.lib.kmb_train_spmd(ctx.handle, _native.KMB_F32 if dt == np.float32 else _native.KMB_F64,
+                                         X.data_ptr(), n, 20, C0.data_ptr(), ctypes.byref(p), ctypes.byref(comm),
+                                         C.data_ptr(), lab.data_ptr(), ctypes.byref(obj), ctypes.byref(it)))
+        return C, lab
+    return run
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("make,n,k", [(_train, 8_000, 40), (_train, 600_000, 300), (_train_sharded, 600_000, 40)],
+                         ids=["small", "update_tail", "sharded"])
+def test_grid_wait_limit_reports_timeout_and_context_recovers(make, n, k, dt, monkeypatch):
+    run = make(dt, n, k, 2)
+    monkeypatch.setenv("KMB_GRID_WAIT_LIMIT_CYCLES", "1")  # the CTAs do not all arrive within a poll
+    with pytest.raises((kmeans.internal_error, _native.NativeError)) as err:
+        run()
+    assert "status 4" in str(err.value)  # KMB_ETIMEDOUT
+    monkeypatch.delenv("KMB_GRID_WAIT_LIMIT_CYCLES")
+    got = run()
+    _native.context(0).lib.kmb_context_release_workspace(_native.context(0).handle)  # state as in a new context
+    for a, b in zip(got, run()):
+        assert torch.equal(a, b)
 
 
 def test_allocation_failure_raises_bad_alloc_and_context_recovers(monkeypatch):
