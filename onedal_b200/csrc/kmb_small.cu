@@ -299,6 +299,97 @@ __device__ __forceinline__ void list_rows(const int *lab, int rows, int k, unsig
     __syncthreads();
 }
 
+// out[0, have): the CTA's rows with the largest d2, in (d2 descending, row ascending) order;
+// 1 <= have <= min(rows, k). A radix select of the have-th row, eight bits a round over the
+// distance's ordered key and then over the row (it ends once a whole bin is taken), the
+// chosen rows listed in any order, and a rank of each in that list. Bound by the reads of d2,
+// a few a row. Comparing every row with every other took 8.2 ms at 12,000 rows a CTA and 3.2 ms at
+// 7,400 (148 CTAs), one empty cluster; 13 and 10 us here. `seg`: kNT ints of scratch.
+template <typename F>
+__device__ void farthest_rows(const F *d2, int rows, int have, int64_t row0, int *seg, SmallCand *out) {
+    static_assert(kNT >= 256 + kSmallTrainMaxK, "bins and chosen rows");
+    int *bins = seg, *chosen = seg + 256;
+    __shared__ int s_bin, s_need, s_all, s_at;
+    constexpr int KD = (int)sizeof(F);  // digits of the key; two more of the row
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int rounds = (rows + kNT - 1) / kNT * kNT;  // (whole warps stay together)
+    unsigned long long key_low = 0;  // the smallest key that can still be the have-th row's
+    unsigned row_low = 0;            // and, at that key, the smallest 0xffff - row
+    int need = have;
+    for (int q = 0; q < KD + 2; ++q) {
+        const int ks = 8 * (KD - 1 - q), rs = 8 * (KD + 1 - q);  // this digit's place in the key, in the row
+        for (int i = tid; i < 256; i += kNT) bins[i] = 0;
+        __syncthreads();
+        for (int r = tid; r < rounds; r += kNT) {
+            bool in = r < rows;
+            unsigned digit = 0;
+            if (in) {
+                const unsigned long long key = key_of(d2[r]);
+                const unsigned inv = 0xffffu - (unsigned)r;
+                if (q < KD) {
+                    in = ((key ^ key_low) >> ks) >> 8 == 0;
+                    digit = (unsigned)(key >> ks) & 0xffu;
+                } else {
+                    in = key == key_low && ((inv ^ row_low) >> rs) >> 8 == 0;
+                    digit = (inv >> rs) & 0xffu;
+                }
+            }
+            const unsigned votes = __ballot_sync(0xffffffffu, in);
+            if (votes == 0) continue;
+            const unsigned first = __shfl_sync(0xffffffffu, digit, __ffs(votes) - 1);
+            if (__all_sync(0xffffffffu, !in || digit == first)) {  // (the leading digits mostly agree)
+                if (lane == 0) atomicAdd(&bins[first], __popc(votes));
+            } else if (in) {
+                atomicAdd(&bins[digit], 1);
+            }
+        }
+        __syncthreads();
+        if (tid < 32) {  // the bin of the need-th row: eight bins a lane, the highest first
+            int c[8], sum = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) sum += c[i] = bins[255 - 8 * lane - i];
+            int before = sum;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, before, o);
+                if (lane >= o) before += t;
+            }
+            before -= sum;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                if (before < need && before + c[i] >= need) {
+                    s_bin = 255 - 8 * lane - i;
+                    s_need = need - before;
+                    s_all = c[i] == need - before;
+                }
+                before += c[i];
+            }
+            if (lane == 0) s_at = 0;
+        }
+        __syncthreads();
+        need = s_need;
+        if (q < KD) key_low |= (unsigned long long)s_bin << ks;
+        else row_low |= (unsigned)s_bin << rs;
+        if (s_all) break;  // (uniform; the next writes of s_* lie behind a barrier)
+    }
+    for (int r = tid; r < rows; r += kNT) {
+        const unsigned long long key = key_of(d2[r]);
+        if (key > key_low || (key == key_low && 0xffffu - (unsigned)r >= row_low)) chosen[atomicAdd(&s_at, 1)] = r;
+    }
+    __syncthreads();
+    for (int e = tid; e < have; e += kNT) {
+        const int r = chosen[e];
+        const unsigned long long key = key_of(d2[r]);
+        int rank = 0;
+        for (int i = 0; i < have; ++i) {
+            const int o = chosen[i];
+            const unsigned long long ok = key_of(d2[o]);
+            rank += ok > key || (ok == key && o < r);
+        }
+        out[rank] = SmallCand{key, (long long)(row0 + r)};
+    }
+}
+
 __device__ __forceinline__ void acc_add(Acc<float> &a, float x, int e) {
     const Limbs L = fixed_of(x, e);
     a.v[0] += L.l0;
@@ -525,18 +616,10 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
         const int ne = __syncthreads_count(tid < k && __ldcg(a.counts + tid) == 0);
         n_empty = ne;
         if (ne > 0) {
-            // this CTA's farthest rows, by rank; then the grid's, by a rank over the CTAs' lists
+            // this CTA's farthest rows in order, then the grid's, by a rank over the CTAs' lists
             const int have = min(ne, rows);
             SmallCand *mine = a.cand + (size_t)b * k;
-            for (int r = tid; r < rows; r += kNT) {
-                const unsigned long long key = key_of(d2[r]);
-                int rank = 0;
-                for (int q = 0; q < rows; ++q) {
-                    const unsigned long long o = key_of(d2[q]);
-                    rank += o > key || (o == key && q < r);
-                }
-                if (rank < have) mine[rank] = SmallCand{key, (long long)(row0 + r)};
-            }
+            farthest_rows(d2, rows, have, row0, seg, mine);
             if (!(ok = grid_sync(sync, arrived, a.wait))) break;
             for (int e = warp; e < have; e += kNW) {
                 const unsigned long long key = __ldcg(&mine[e].key);

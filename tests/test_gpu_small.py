@@ -4,8 +4,11 @@ exact, so that both give the same responses. Sizes at the edges of the rule and 
 kernel: one CTA and many, ragged rows per CTA, the padded column counts, one cluster, as
 many clusters as threads allow, fewer rows than clusters would fill, empty clusters over
 several CTAs."""
+import time
+
 import numpy as np
 import pytest
+import torch
 
 from onedal_b200 import kmeans
 from oracle import restated
@@ -63,6 +66,45 @@ def test_empty_clusters_take_the_farthest_rows_over_all_blocks():
     order = np.lexsort((np.arange(n), -(X ** 2).sum(1)))[:k - 1]
     np.testing.assert_array_equal(r.get_model().get_centroids()[1:], X[order])
     assert r.stats.empty_cluster_events == k - 1
+
+
+@pytest.mark.parametrize("dt,n,d,k,span", [(np.float32, 1_100_000, 3, 200, 300), (np.float32, 1_100_000, 3, 200, 2),
+                                           (np.float64, 1_050_000, 1, 100, 10**6), (np.float32, 1_050_000, 1, 256, 0),
+                                           (np.float64, 2000, 1, 256, 9)])
+def test_empty_clusters_take_the_farthest_of_many_rows_per_block(dt, n, d, k, span):
+    """Thousands of rows in a block, all but one cluster empty: distances that differ, that tie
+    in their thousands, and that are all the same (the lowest rows then)."""
+    rng = np.random.default_rng(span)
+    X = rng.integers(-span, span + 1, (n, d)).astype(dt) + 1
+    C0 = np.full((k, d), 1e9, dt)
+    C0[0] = 0
+    desc = kmeans.descriptor(dt).set_cluster_count(k).set_max_iteration_count(1)
+    r = kmeans.train(desc.set_compute_form(kmeans.compute_form.plain), X, C0)
+    order = np.lexsort((np.arange(n), -(X.astype(np.float64) ** 2).sum(1)))[:k - 1]
+    np.testing.assert_array_equal(r.get_model().get_centroids()[1:], X[order])
+
+
+@pytest.mark.parametrize("dt,n,d,k", [(np.float32, 1_100_000, 3, 200), (np.float64, 1_050_000, 1, 100)])
+def test_an_empty_cluster_costs_no_more_than_the_iteration(dt, n, d, k):
+    """The selection reads the distances a few times; ranking rows against rows took six
+    trains' time."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    X = torch.randn(n, d, device="cuda", generator=g, dtype=torch.float32 if dt == np.float32 else torch.float64)
+    desc = kmeans.descriptor(dt).set_cluster_count(k).set_max_iteration_count(1)
+    desc.set_compute_form(kmeans.compute_form.plain)
+    times = []
+    for empty in (0, 1):
+        C = X[:k].clone()
+        if empty:
+            C[-1] = 1e6
+        assert kmeans.train(desc, X, C).stats.empty_cluster_events == empty
+        runs = []
+        for _ in range(9):
+            t = time.perf_counter()
+            kmeans.train(desc, X, C)
+            runs.append(time.perf_counter() - t)
+        times.append(sorted(runs)[4])
+    assert times[1] < 2 * times[0], times
 
 
 @pytest.mark.parametrize("span", [1, 40, 80, 120])
