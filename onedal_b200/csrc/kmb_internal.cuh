@@ -307,7 +307,8 @@ void launch_update(const F *X, const UpdatePlan &p, const int32_t *labels, const
                    F *exact_d2 = nullptr);
 
 // ---- small dense problems (plain form): the whole train in one cooperative launch ----
-// Taken when the rows fit the SMs' shared memory, k <= 256, d <= 64 and n * k * d <= 2^30:
+// Taken when the rows fit the SMs' shared memory, k <= 256, d <= 64 and n * k * d <= 2^30
+// (but for wide problems of few rows, see make_small_plan):
 // up to there an iteration's arithmetic is no longer than the 14 launches of the general
 // path (30 us); 100,000 x 20, k = 20 takes 19 us an iteration here and 68 us there.
 constexpr int64_t kSmallTrainMaxK = 256;

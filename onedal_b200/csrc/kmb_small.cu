@@ -18,7 +18,7 @@
 //               added in order: float values as the exact integers of the exact update,
 //               double values in FP64 in a fixed order
 //   barrier
-//   finalize    one warp per (cluster, column) over the grid: the CTAs' sums in a fixed
+//   finalize    as many lanes per (cluster, column) as CTAs, over the grid: their sums in a fixed
 //               order, the new centroid value and its part of the shift
 //   barrier
 //   decide      every CTA reads the new centroids, counts and shift parts and takes the
@@ -495,6 +495,10 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
     const int nseg = small_segments(d);
     const int seg_rows = (rows + nseg - 1) / nseg;
     const bool runs = a.runs != 0;
+    // the finalize takes 2^lg lanes a cell: as many as there are CTAs, a warp at most
+    int lg = 0;
+    while (lg < 5 && 1 << lg < G) ++lg;
+    const int sub = lane & ((1 << lg) - 1), slot = lane >> lg;
     while (ok && !done && iterations < a.T) {
         assign_rows<F, DMAX>(Xs, ds, Cs, hs, xn, rows, d, k, lab, d2);
         __syncthreads();
@@ -567,21 +571,24 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
         }
         for (int j = tid; j < k; j += kNT) a.part_cnt[(size_t)j * G + b] = start[j + 1] - start[j];
         if (!(ok = grid_sync(sync, arrived, a.wait))) break;
-        // finalize: one warp per cell over the grid
-        for (int cell = b * kNW + warp; cell < cells; cell += G * kNW) {
-            const int j = cell / d, t = cell - j * d;
+        // finalize over the grid (256 x 64, k = 256, one CTA: 1460 us a train with a warp per
+        // cell, 235 us with a thread)
+        for (int first = (b * kNW + warp) << (5 - lg); first < cells; first += (G * kNW) << (5 - lg)) {
+            const int cell = first + slot;
+            const bool in = cell < cells;
+            const int j = in ? cell / d : 0, t = in ? cell - j * d : 0;
             Acc<F> s = {};
             int cnt = 0;
-            for (int c0 = lane; c0 < G; c0 += 5 * 32) {  // five CTAs' loads in flight per lane
+            for (int c0 = sub; c0 < G; c0 += 5 * 32) {  // five CTAs' loads in flight per lane
                 unsigned long long v[5][NP];
                 int n5[5];
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {
                     const int c = c0 + 32 * q;
-                    n5[q] = c < G ? __ldcg(a.part_cnt + (size_t)j * G + c) : 0;
+                    n5[q] = in && c < G ? __ldcg(a.part_cnt + (size_t)j * G + c) : 0;
 #pragma unroll
                     for (int l = 0; l < NP; ++l)
-                        v[q][l] = c < G ? __ldcg(a.part + ((size_t)l * cells + cell) * G + c) : 0ull;  // (0.0 too)
+                        v[q][l] = in && c < G ? __ldcg(a.part + ((size_t)l * cells + cell) * G + c) : 0ull;  // (0.0 too)
                 }
 #pragma unroll
                 for (int q = 0; q < 5; ++q) {
@@ -590,12 +597,14 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
                     for (int l = 0; l < NP; ++l) s.v[l] += *reinterpret_cast<const decltype(s.v[0] + 0) *>(&v[q][l]);
                 }
             }
+#pragma unroll
             for (int m = 16; m >= 1; m >>= 1) {
+                if (m >> lg) continue;
 #pragma unroll
                 for (int l = 0; l < NP; ++l) s.v[l] += __shfl_xor_sync(0xffffffffu, s.v[l], m);
                 cnt += __shfl_xor_sync(0xffffffffu, cnt, m);
             }
-            if (lane == 0) {
+            if (in && sub == 0) {
                 const F old = Cs[j * DMAX + t];
                 const F c = cnt > 0 ? centroid_of(s, sizeof(F) == 4 ? s_exp[t] : 0, cnt) : old;
                 const double df = (double)old - (double)c;
@@ -742,10 +751,24 @@ SmallPlan make_small_plan(int64_t n, int64_t d, int64_t k) {
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     optin -= 2048;  // static shared memory
-    // one CTA while it does an iteration's work in the time that barriers and the exchange
-    // would take (about 10,000 cycles), else blocks of at least 256 rows over the SMs
-    const int64_t one_cta_macs = sizeof(F) == 4 ? 1 << 20 : 1 << 19;
-    int64_t ctas = n * k * d <= one_cta_macs ? 1 : std::min<int64_t>(sms, (n + 255) / 256);
+    // A row's k * d products are one thread's work, so a wide problem of few rows leaves most of
+    // the chip idle here, and the general path is the better one (train of 10 iterations there
+    // and here, us): floats and doubles of d <= 32, whose row is in registers, 1000 x 64, k = 256
+    // 519 and 820, 4000 x 64, k = 256 502 and 490, 1000 x 64, k = 160 460 and 448; wider doubles
+    // 4000 x 48, k = 128 503 and 399, 4000 x 64, k = 128 565 and 638, k = 256 570 and 982.
+    const int64_t kd = k * d;
+    if (sizeof(F) * dmax <= 256 ? kd > 10240 && n < 4096 : kd > 6144) return p;
+    // One CTA of at most a row per thread while it does an iteration's work in about the time
+    // that barriers and the exchange take (300 x 1, k = 3 113 us, in two CTAs 125; 400 x 64,
+    // k = 10 149 and 126). Else blocks of 256 rows over the SMs, or, up to 125 CTAs, of fewer
+    // rows, 2^19 multiply-adds an iteration but 64 rows at least (3000 x 60, k = 100 361 us by
+    // 256 rows, 287 by 87; past 125 the exchange outweighs: 8000 x 64, k = 256 460 us in 125
+    // CTAs, 496 in 148; and 32,000 x 64, k = 256 1140 us in 125, 1340 in 128, whose strides of
+    // 1 KB fall on few L2 slices).
+    const int64_t light = std::max<int64_t>(64, (1 << 19) / kd);
+    int64_t ctas = 1;
+    if (n > kNT || n * kd > 1 << 17)
+        ctas = std::min<int64_t>(sms, std::max((n + 255) / 256, std::min<int64_t>(125, (n + light - 1) / light)));
     for (;;) {
         const int64_t rows = (n + ctas - 1) / ctas;
         if (rows <= 65535 && small_layout<F>((int)rows, (int)d, (int)k, dmax).total <= (size_t)optin) {

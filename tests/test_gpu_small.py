@@ -30,7 +30,11 @@ def _data(n, d, k, dt, seed, dup):
 @pytest.mark.parametrize("n,d,k,T,dup", [(1, 1, 1, 3, False), (100, 3, 3, 50, False), (513, 4, 2, 20, False),
                                          (2047, 24, 7, 20, True), (2049, 33, 40, 10, True), (30_001, 20, 20, 12, False),
                                          (9_999, 64, 256, 6, True), (148 * 256 + 1, 8, 33, 9, True),
-                                         (60_000, 47, 61, 5, False)])
+                                         (60_000, 47, 61, 5, False),
+                                         # the edges of the rule: one CTA or more, rows per CTA, the general path
+                                         (512, 16, 16, 8, True), (512, 16, 17, 8, False), (4096, 64, 161, 5, True),
+                                         (4095, 64, 161, 5, False), (1025, 64, 160, 5, True), (3000, 32, 256, 5, False),
+                                         (2500, 33, 186, 5, True), (2500, 33, 187, 5, False)])
 def test_equals_the_general_path(dt, n, d, k, T, dup):
     X, C0 = _data(n, d, k, dt, n + d + k, dup)
     desc = kmeans.descriptor(dt).set_cluster_count(k).set_max_iteration_count(T)
@@ -105,6 +109,26 @@ def test_an_empty_cluster_costs_no_more_than_the_iteration(dt, n, d, k):
             runs.append(time.perf_counter() - t)
         times.append(sorted(runs)[4])
     assert times[1] < 2 * times[0], times
+
+
+@pytest.mark.parametrize("dt", [np.float32, np.float64])
+@pytest.mark.parametrize("n,d,k", [(256, 64, 256), (400, 64, 256), (1000, 64, 256), (4000, 64, 256), (12_000, 1, 80)])
+def test_no_slower_than_the_general_path(dt, n, d, k):
+    """The general path is asked for with the recheck, which it pays for as well."""
+    g = torch.Generator(device="cuda").manual_seed(1)
+    X = torch.randn(n, d, device="cuda", generator=g, dtype=torch.float32 if dt == np.float32 else torch.float64)
+    C = X[:k].clone()
+    times = []
+    for recheck in (False, True):
+        desc = kmeans.descriptor(dt).set_cluster_count(k).set_max_iteration_count(10)
+        desc.set_compute_form(kmeans.compute_form.plain).set_recheck(recheck)
+        runs = []
+        for _ in range(13):
+            t = time.perf_counter()
+            kmeans.train(desc, X, C)
+            runs.append(time.perf_counter() - t)
+        times.append(sorted(runs)[6])
+    assert times[0] < 1.25 * times[1], times
 
 
 @pytest.mark.parametrize("span", [1, 40, 80, 120])
