@@ -169,11 +169,6 @@ cudaError_t allow_smem(const void *kern) {
     return e;
 }
 
-std::mutex &cooperative_mutex() {
-    static std::mutex mu;
-    return mu;
-}
-
 // From the library's pool when it exists, else the device's default pool.
 cudaError_t pool_alloc(void **p, size_t bytes, int dev, cudaStream_t s) {
     cudaMemPool_t pool = library_pool(dev);
@@ -539,7 +534,7 @@ int run_loop(kmb_context *ctx, const F *X, int64_t n, int64_t d, F *C, const kmb
 }
 
 // A small problem's train (or its iterations only) in one launch; waits for it and leaves
-// its state in h_state[0]. The lock is taken for the launch's whole time on the device.
+// its state in h_state[0].
 template <typename F>
 int run_small(kmb_context *ctx, const kmb::SmallPlan &plan, const F *X, int64_t n, int64_t d, const F *C0,
               const kmb_params *p, bool final_pass, F *C_out, int32_t *labels) {
@@ -550,7 +545,6 @@ int run_small(kmb_context *ctx, const kmb::SmallPlan &plan, const F *X, int64_t 
         return fail(ctx, KMB_ENOMEM, "device allocation failed (n=%lld d=%lld k=%lld)", (long long)n, (long long)d,
                     (long long)p->cluster_count);
     ProfRange range("kmb_small_train");
-    std::lock_guard<std::mutex> lock(kmb::cooperative_mutex());
     {
         KernelTimer timer(ctx, 0);
         KMB_CUDA(kmb::launch_small_train<F>(plan, X, n, d, C0, p->cluster_count, p->max_iteration_count,

@@ -1213,7 +1213,6 @@ extern "C" int kmb_batched_train(int dtype, kmb_batched_problem *problems, int64
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     bool graphed = false;
-    std::unique_lock<std::mutex> lock(cooperative_mutex());  // until the grid has ended
     // device time of the kernel alone (host set-up excluded)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     const bool timed = cudaEventCreate(&ev0) == cudaSuccess && cudaEventCreate(&ev1) == cudaSuccess;
@@ -1250,7 +1249,6 @@ extern "C" int kmb_batched_train(int dtype, kmb_batched_problem *problems, int64
                          cudaMemcpyAsync(&hb, gb, sizeof(hb), cudaMemcpyDeviceToHost, s) != cudaSuccess))
         rc = KMB_ECUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess || cudaGetLastError() != cudaSuccess) rc = KMB_ECUDA;
-    lock.unlock();
     if (rc == KMB_OK && hb.error) rc = hb.error == 1 ? KMB_ETIMEDOUT : KMB_ECUDA;
     if (rc == KMB_OK) {
         long long total_iters = 0;

@@ -5,7 +5,6 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-#include <mutex>
 #include <string>
 
 #include "../../include/onedal_b200_kmeans.h"
@@ -56,8 +55,10 @@ constexpr long long kGridTimeout = 4000000000ll;  // ~2 s of SM clocks per wait
 // environment (tests make a wait run out).
 long long grid_wait_cycles();
 
-// Every CTA of the grid arrives before any leaves (cooperative launch: all CTAs are
-// resident); `arrived` counts this CTA's barriers, from zero. One release-add and acquire
+// Every CTA of the grid arrives before any leaves. Only for cooperative launches, whose CTAs
+// the runtime keeps resident together whatever else runs on the device; so launches of this
+// kind need no order among themselves, and no lock of the host's.
+// `arrived` counts this CTA's barriers, from zero. One release-add and acquire
 // polls of a count that only grows: about 1500 cycles, where a barrier with a generation
 // word, a reset and full fences took 5000. The wait is bounded by `limit` cycles; false when
 // this CTA's ran out, which is recorded in sy->error (the others' then run out too; the
@@ -328,16 +329,10 @@ struct SmallOut {
 };
 // C0 (k x d) -> C_out (k x d; may be C0), labels (n, may be null) and the SmallOut at the
 // start of scratch. final_pass: the labels are those under the final centroids and
-// st.objective is set; else they are the last update's. The grid's CTAs wait for one another: launches that do are kept apart by
-// cooperative_mutex until they have ended.
+// st.objective is set; else they are the last update's.
 template <typename F>
 cudaError_t launch_small_train(const SmallPlan &p, const F *X, int64_t n, int64_t d, const F *C0, int64_t k, int64_t T,
                                double eps, bool final_pass, F *C_out, int32_t *labels, void *scratch, cudaStream_t s);
-// Held by a host thread from a launch that may fill the device with CTAs waiting for one
-// another until that launch has ended, so that two such grids are never partly resident
-// at a time.
-std::mutex &cooperative_mutex();
-
 // ---- exact fixed-point sums (shared by the Lloyd update and the batched form) ----
 // A value x of column t is the integer v = round(x * 2^E_t), |v| < 2^94, E_t =
 // 94 - (exponent of the column's largest |x|); v is handled as three 32-bit

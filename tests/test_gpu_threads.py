@@ -1,7 +1,9 @@
 """Calls from several host threads, a context each: every call's result is the one that it
 gives alone. Each pair of jobs reaches one kernel with different amounts of dynamic shared
-memory, whose limit is an attribute that the threads share."""
+memory, whose limit is an attribute that the threads share. And no thread's small train waits
+for another's long one."""
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -103,3 +105,34 @@ def test_threads_get_what_they_get_alone(make):
     for t in threads:
         t.join()
     assert not wrong, wrong[:3]
+
+
+@pytest.mark.parametrize("n", [100, 2000], ids=["one_block", "blocks"])
+def test_a_small_train_does_not_wait_for_another_threads(n):
+    """A train of eight blocks that never converges (a NaN in its rows) runs for its 20,000
+    iterations; a thread with a few blocks' train, which the other SMs can hold, is done long
+    before."""
+    def args(n, T):
+        X, C = _rows(n, 20, 20)
+        desc = kmeans.descriptor(np.float32).set_cluster_count(20).set_max_iteration_count(T)
+        return desc.set_compute_form(kmeans.compute_form.plain), X, C
+    long_args, short_args = args(2001, 20_000), args(n, 3)
+    long_args[1][5, 5] = float("nan")
+    kmeans.train(*short_args)
+    ended = {}
+
+    def work(name, a):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            kmeans.train(*a)
+        ended[name] = time.perf_counter()
+
+    threads = [threading.Thread(target=work, args=("long", long_args)), threading.Thread(target=work, args=("short", short_args))]
+    torch.cuda.synchronize()
+    t0 = time.perf_counter()
+    threads[0].start()
+    time.sleep(0.03)
+    threads[1].start()
+    for t in threads:
+        t.join()
+    assert ended["long"] - t0 > 0.15, "the long train was over before the other began"
+    assert ended["long"] - ended["short"] > 0.05, ended
