@@ -77,7 +77,7 @@ __device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived, long 
         int ok = 1;
         for (;;) {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(&sy->count) : "memory");
-            if (seen >= target) break;
+            if ((int)(seen - target) >= 0) break;  // (the count wraps in a long enough loop)
             if (clock64() - t0 > limit) {
                 atomicExch(&sy->error, 1);
                 ok = 0;
