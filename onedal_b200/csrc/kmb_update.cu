@@ -532,6 +532,16 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
         }
     }
     if (!grid_sync(sy, arrived, wait)) return false;
+    int P = 1, lg = 0;
+    while (P < m) {
+        P <<= 1;
+        ++lg;
+    }
+    // The other CTAs' last wait allows for CTA 0's work alone, at 4096 cycles a step of
+    // kTailThreads entries: up to n / kTailThreads steps in search of equal rows, and lg (lg +
+    // 1) / 2 passes of a sort in global memory (65,535 candidates 6.9 ms).
+    static_assert(kTailThreads == 512, "8 cycles an entry");
+    const long long serial = (all_eq ? 0ll : 8ll * n) + (P <= kSortSmem ? 0ll : 4ll * P * lg * (lg + 1));
     if (blockIdx.x == 0) {
         if (!all_eq) {
             if (tid == 0) s_base = (unsigned)m - need;
@@ -556,8 +566,6 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
                 __syncthreads();
             }
         }
-        int P = 1;
-        while (P < m) P <<= 1;
         if (P <= kSortSmem) {
             for (int i = tid; i < P; i += kTailThreads) {
                 Cand e{0ull, 0x7fffffffffffffffll};
@@ -576,7 +584,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
             cand_sort(cand, P);
         }
     }
-    return grid_sync(sy, arrived, wait);
+    return grid_sync(sy, arrived, wait + serial);
 }
 
 // Exact squared distances for the empty-cluster candidates: when some cluster is

@@ -44,3 +44,18 @@ def test_empty_clusters_take_the_farthest_rows(dt, n, m, span):
     dist = (X.astype(np.int64) ** 2).sum(1)
     order = np.lexsort((np.arange(n), -dist))[:m]
     np.testing.assert_array_equal(out[1:], X[order])
+
+
+def test_one_blocks_sort_outlasts_a_wait(monkeypatch):
+    """65,535 empty clusters: one block sorts the candidates while the others wait, longer than
+    the limit of an ordinary wait (lowered here to 2 ms); their wait allows for it."""
+    n, m, d = 70_000, 65_535, 3
+    rng = np.random.default_rng(9)
+    X = rng.integers(-200, 201, (n, d)).astype(np.float32)
+    C = np.zeros((m + 1, d), np.float32)
+    C[1:] = 10000.0
+    monkeypatch.setenv("KMB_GRID_WAIT_LIMIT_CYCLES", "4000000")
+    out, lab, ne = _step(X, C)
+    assert ne == m and (lab == 0).all()
+    order = np.lexsort((np.arange(n), -(X.astype(np.int64) ** 2).sum(1)))[:m]
+    np.testing.assert_array_equal(out[1:], X[order])
