@@ -552,6 +552,7 @@ int run_small(kmb_context *ctx, const kmb::SmallPlan &plan, const F *X, int64_t 
     }
     KMB_CUDA(cudaMemcpyAsync(ctx->h_state, ws.small.ptr, sizeof(kmb::SmallOut), cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaStreamSynchronize(s));
+    ctx->queue_state = nullptr;  // this call queued no rows (kmb_context_recheck_rows)
     if (reinterpret_cast<const kmb::SmallOut *>(ctx->h_state)->sync.error)
         return fail(ctx, KMB_ETIMEDOUT, "device loop failed (status %d)", KMB_ETIMEDOUT);
     return KMB_OK;

@@ -4,13 +4,14 @@ exact, so that both give the same responses. Sizes at the edges of the rule and 
 kernel: one CTA and many, ragged rows per CTA, the padded column counts, one cluster, as
 many clusters as threads allow, fewer rows than clusters would fill, empty clusters over
 several CTAs."""
+import ctypes
 import time
 
 import numpy as np
 import pytest
 import torch
 
-from onedal_b200 import kmeans
+from onedal_b200 import _native, kmeans
 from oracle import restated
 
 pytestmark = pytest.mark.gpu
@@ -167,3 +168,24 @@ def test_infinite_rows_take_the_same_sums_as_the_general_path():
     a = kmeans.train(desc, X, X[10:15].copy())
     b = kmeans.train(desc.set_recheck(True), X, X[10:15].copy())
     np.testing.assert_array_equal(a.get_model().get_centroids(), b.get_model().get_centroids())
+
+
+def _train_args(n=5000, d=20, k=20, T=4):
+    X, C0 = _data(n, d, k, np.float32, 7, False)
+    desc = kmeans.descriptor(np.float32).set_cluster_count(k).set_max_iteration_count(T)
+    return desc.set_compute_form(kmeans.compute_form.plain), torch.from_numpy(X).cuda(), torch.from_numpy(C0).cuda()
+
+
+def test_a_train_without_recheck_leaves_no_rechecked_rows():
+    """kmb_context_recheck_rows is about the context's last pass, not an earlier call's."""
+    ctx = _native.context(0)
+    desc, X, C = _train_args()
+    tied = torch.cat([C, C])  # every row's two nearest clusters tie
+    tc = kmeans.descriptor(np.float32).set_cluster_count(40).set_compute_form(kmeans.compute_form.bf16x3)
+    kmeans.infer(tc, kmeans.model(tied), X)
+    count = ctypes.c_int64()
+    ctx.check(ctx.lib.kmb_context_recheck_rows(ctx.handle, None, 0, ctypes.byref(count)))
+    assert count.value == X.shape[0]
+    kmeans.train(desc, X, C)
+    ctx.check(ctx.lib.kmb_context_recheck_rows(ctx.handle, None, 0, ctypes.byref(count)))
+    assert count.value == 0
