@@ -268,7 +268,8 @@ KMB_API int kmb_lloyd_iterate(kmb_context *ctx, int dtype, const void *X, int64_
  * read (synchronising) with kmb_context_kernel_time and cleared by enabling
  * again. kernel: 0 = plain assignment, 1 = tensor-core assignment, 2 = update,
  * 4 = FP64 near-tie recheck; kernel 3 returns in *launches every kernel this
- * host thread launched since timing was enabled (total_ms = 0). */
+ * host thread launched since timing was enabled (total_ms = 0). Small trains,
+ * otherwise one launch, run as these separate kernels while timing is on. */
 KMB_API int kmb_context_set_kernel_timing(kmb_context *ctx, int enabled);
 /* Grid of the persistent launches (tensor-core assignment, row splitting,
  * recheck): at most max_sms SMs (0: all), leaving the rest to other streams'

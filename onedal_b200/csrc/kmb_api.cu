@@ -533,6 +533,13 @@ int run_loop(kmb_context *ctx, const F *X, int64_t n, int64_t d, F *C, const kmb
     return KMB_OK;
 }
 
+// The one-launch train is for the plain form without recheck; with kernel timing on, the
+// separate kernels are what the caller asks about.
+template <typename F>
+kmb::SmallPlan small_plan(const kmb_context *ctx, int64_t n, int64_t d, int64_t k, bool recheck) {
+    return recheck || ctx->timing ? kmb::SmallPlan() : kmb::make_small_plan<F>(n, d, k);
+}
+
 // A small problem's train (or its iterations only) in one launch; waits for it and leaves
 // its state in h_state[0].
 template <typename F>
@@ -545,11 +552,8 @@ int run_small(kmb_context *ctx, const kmb::SmallPlan &plan, const F *X, int64_t 
         return fail(ctx, KMB_ENOMEM, "device allocation failed (n=%lld d=%lld k=%lld)", (long long)n, (long long)d,
                     (long long)p->cluster_count);
     ProfRange range("kmb_small_train");
-    {
-        KernelTimer timer(ctx, 0);
-        KMB_CUDA(kmb::launch_small_train<F>(plan, X, n, d, C0, p->cluster_count, p->max_iteration_count,
-                                            p->accuracy_threshold, final_pass, C_out, labels, ws.small.ptr, s));
-    }
+    KMB_CUDA(kmb::launch_small_train<F>(plan, X, n, d, C0, p->cluster_count, p->max_iteration_count,
+                                        p->accuracy_threshold, final_pass, C_out, labels, ws.small.ptr, s));
     KMB_CUDA(cudaMemcpyAsync(ctx->h_state, ws.small.ptr, sizeof(kmb::SmallOut), cudaMemcpyDeviceToHost, s));
     KMB_CUDA(cudaStreamSynchronize(s));
     ctx->queue_state = nullptr;  // this call queued no rows (kmb_context_recheck_rows)
@@ -566,7 +570,7 @@ int iterate_impl(kmb_context *ctx, const void *Xv, int64_t n, int64_t d, void *C
     ctx->tc_products = form_products(p->form);
     if (tc && !kmb::tc_supported(d)) return fail(ctx, KMB_EUNSUPPORTED, "tensor-core form needs d <= 256");
     const bool recheck = p->recheck != 0 || tc;
-    const kmb::SmallPlan small = recheck ? kmb::SmallPlan() : kmb::make_small_plan<F>(n, d, k);
+    const kmb::SmallPlan small = small_plan<F>(ctx, n, d, k, recheck);
     if (small.ctas) {
         int rc = run_small<F>(ctx, small, (const F *)Xv, n, d, (const F *)Cv, p, false, (F *)Cv, labels);
         if (rc) return rc;
@@ -609,7 +613,7 @@ int train_impl(kmb_context *ctx, int memory, const void *Xv, int64_t n, int64_t 
     ctx->tc_products = form_products(p->form);
     if (tc && !kmb::tc_supported(d)) return fail(ctx, KMB_EUNSUPPORTED, "tensor-core form needs d <= 256");
     const bool recheck = p->recheck != 0 || tc;
-    const kmb::SmallPlan small = recheck ? kmb::SmallPlan() : kmb::make_small_plan<F>(n, d, k);
+    const kmb::SmallPlan small = small_plan<F>(ctx, n, d, k, recheck);
     int rc;
     kmb::UpdatePlan plan;
     if (!small.ctas) {

@@ -176,6 +176,27 @@ def _train_args(n=5000, d=20, k=20, T=4):
     return desc.set_compute_form(kmeans.compute_form.plain), torch.from_numpy(X).cuda(), torch.from_numpy(C0).cuda()
 
 
+def test_kernel_times_are_still_told_apart():
+    """With kernel timing on, a train's assignments and updates are timed one by one."""
+    ctx = _native.context(0)
+    args = _train_args()
+    alone = kmeans.train(*args)
+    ctx.check(ctx.lib.kmb_context_set_kernel_timing(ctx.handle, 1))
+    try:
+        timed = kmeans.train(*args)
+        ms, launches = ctypes.c_double(), ctypes.c_int64()
+        counts = {}
+        for kernel in (0, 2):
+            ctx.check(ctx.lib.kmb_context_kernel_time(ctx.handle, kernel, ctypes.byref(ms), ctypes.byref(launches)))
+            counts[kernel] = launches.value
+            assert ms.value > 0
+    finally:
+        ctx.check(ctx.lib.kmb_context_set_kernel_timing(ctx.handle, 0))
+    assert counts == {0: 5, 2: 4}
+    assert torch.equal(alone.get_model().get_centroids(), timed.get_model().get_centroids())
+    assert torch.equal(alone.get_responses(), timed.get_responses())
+
+
 def test_a_train_without_recheck_leaves_no_rechecked_rows():
     """kmb_context_recheck_rows is about the context's last pass, not an earlier call's."""
     ctx = _native.context(0)
