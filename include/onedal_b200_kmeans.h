@@ -272,7 +272,7 @@ KMB_API int kmb_lloyd_iterate(kmb_context *ctx, int dtype, const void *X, int64_
  * otherwise one launch, run as these separate kernels while timing is on. */
 KMB_API int kmb_context_set_kernel_timing(kmb_context *ctx, int enabled);
 /* Grid of the persistent launches (tensor-core assignment, row splitting,
- * recheck): at most max_sms SMs (0: all), leaving the rest to other streams'
+ * recheck, small trains): at most max_sms SMs (0: all), leaving the rest to other streams'
  * work. max_sms = -1 instead launches the tensor-core assignment as one short
  * CTA per 128-row tile, which other streams' launches interleave with at tile
  * granularity -- the serving loop uses it so that neither side waits for a

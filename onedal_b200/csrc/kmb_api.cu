@@ -534,10 +534,10 @@ int run_loop(kmb_context *ctx, const F *X, int64_t n, int64_t d, F *C, const kmb
 }
 
 // The one-launch train is for the plain form without recheck; with kernel timing on, the
-// separate kernels are what the caller asks about.
+// separate kernels are what the caller asks about. Its grid keeps to the context's SMs.
 template <typename F>
 kmb::SmallPlan small_plan(const kmb_context *ctx, int64_t n, int64_t d, int64_t k, bool recheck) {
-    return recheck || ctx->timing ? kmb::SmallPlan() : kmb::make_small_plan<F>(n, d, k);
+    return recheck || ctx->timing ? kmb::SmallPlan() : kmb::make_small_plan<F>(n, d, k, ctx->num_sms);
 }
 
 // A small problem's train (or its iterations only) in one launch; waits for it and leaves

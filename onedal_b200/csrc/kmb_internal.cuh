@@ -319,7 +319,7 @@ struct SmallPlan {
     int rows = 0;  // per CTA
 };
 template <typename F>
-SmallPlan make_small_plan(int64_t n, int64_t d, int64_t k);
+SmallPlan make_small_plan(int64_t n, int64_t d, int64_t k, int sms);  // sms: CTAs at most
 template <typename F>
 size_t small_scratch_bytes(const SmallPlan &p, int64_t d, int64_t k);
 // What a small train leaves: valid unless sync.error is set.

@@ -742,14 +742,13 @@ const void *kernel_of(int dmax) {
 }  // namespace
 
 template <typename F>
-SmallPlan make_small_plan(int64_t n, int64_t d, int64_t k) {
+SmallPlan make_small_plan(int64_t n, int64_t d, int64_t k, int sms) {
     SmallPlan p;
     const int dmax = dmax_of(d);
     if (dmax == 0 || k > kSmallTrainMaxK || n > INT32_MAX || n * k * d > kSmallTrainMacs) return p;
-    int dev = 0, optin = 0, sms = 148;
+    int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     optin -= 2048;  // static shared memory
     // A row's k * d products are one thread's work, so a wide problem of few rows leaves most of
     // the chip idle here, and the general path is the better one (train of 10 iterations there
@@ -841,7 +840,7 @@ cudaError_t launch_small_train(const SmallPlan &p, const F *X, int64_t n, int64_
 }
 
 #define KMB_SMALL_INST(F)                                                                                             \
-    template SmallPlan make_small_plan<F>(int64_t, int64_t, int64_t);                                                 \
+    template SmallPlan make_small_plan<F>(int64_t, int64_t, int64_t, int);                                               \
     template size_t small_scratch_bytes<F>(const SmallPlan &, int64_t, int64_t);                                      \
     template cudaError_t launch_small_train<F>(const SmallPlan &, const F *, int64_t, int64_t, const F *, int64_t,    \
                                                int64_t, double, bool, F *, int32_t *, void *, cudaStream_t);

@@ -5,6 +5,7 @@ kernel: one CTA and many, ragged rows per CTA, the padded column counts, one clu
 many clusters as threads allow, fewer rows than clusters would fill, empty clusters over
 several CTAs."""
 import ctypes
+import json
 import time
 
 import numpy as np
@@ -210,3 +211,23 @@ def test_a_train_without_recheck_leaves_no_rechecked_rows():
     kmeans.train(desc, X, C)
     ctx.check(ctx.lib.kmb_context_recheck_rows(ctx.handle, None, 0, ctypes.byref(count)))
     assert count.value == 0
+
+
+def test_grid_stays_within_the_contexts_sms(tmp_path):
+    """kmb_context_set_max_sms bounds the grid of this persistent launch too."""
+    from torch.profiler import ProfilerActivity, profile
+    ctx = _native.context(0)
+    args = _train_args()
+    alone = kmeans.train(*args)
+    ctx.check(ctx.lib.kmb_context_set_max_sms(ctx.handle, 3))
+    try:
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            few = kmeans.train(*args)
+            torch.cuda.synchronize()
+    finally:
+        ctx.check(ctx.lib.kmb_context_set_max_sms(ctx.handle, 0))
+    p.export_chrome_trace(str(tmp_path / "trace.json"))
+    events = json.load(open(tmp_path / "trace.json"))["traceEvents"]
+    grids = [e["args"]["grid"][0] for e in events if "small_train_kernel" in e.get("name", "")]
+    assert grids and max(grids) <= 3, grids
+    assert torch.equal(alone.get_model().get_centroids(), few.get_model().get_centroids())
