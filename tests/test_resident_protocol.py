@@ -2,13 +2,12 @@
 checked on the CPU before any GPU runs it.
 
 The kernel's two warp groups take turns at the FMA pipe through named barriers 1 and
-2, meet at CTA barriers around each chunk's centroid load, at a group barrier after a
-tile's last contraction (one-stage form), and consume TMA row loads in the order their
-single issuing thread issued them. The model replays each group's sequence of those
+2, meet at a group barrier after a tile's last contraction (one-stage form), and consume
+TMA row loads in the order their single issuing thread issued them. The model replays each group's sequence of those
 operations for one CTA -- the same loop bounds, tile indices, next-tile rule, stage and
 parity bookkeeping as the kernel -- and schedules the two groups against each other.
 It checks, for row counts around the tile and step sizes, grids that wrap, one or
-several chunks, one or two stages and several block sizes:
+several passes, and one or two stages:
 
 * no deadlock: every turn wait is matched by the other group's hand-over, with never
   more than one hand-over pending on a barrier (a second arrival would complete the
@@ -22,65 +21,47 @@ import pytest
 R = 64  # rows per tile
 
 
-def group_program(g, n, grid, b, kres, kchunk, bt, stages):
+def group_program(g, n, grid, b, kres, stages):
     n_tiles = (n + R - 1) // R
     par_tiles = (n_tiles - g + 1) // 2
     par_tiles0 = (n_tiles + 1) // 2
     my_tiles = (par_tiles - b + grid - 1) // grid if par_tiles > b else 0
     steps = (par_tiles0 - b + grid - 1) // grid if par_tiles0 > b else 0
-    n_chunks = (kres + kchunk - 1) // kchunk
-    total_turns = steps * (kres // 256)
-    ops, m_issue, m_wait, turn = [], 0, 0, 0
+    passes = kres // 256
+    total_turns = steps * passes
+    ops, turn = [], 0
     if my_tiles > 0:
         ops.append(("issue", 0, 0))
-        m_issue = 1
-    for blk in range((steps + bt - 1) // bt):
-        u_n = min(bt, steps - blk * bt)
-        for q in range(n_chunks):
-            if n_chunks > 1 and (blk > 0 or q > 0):
-                ops += [("cta",), ("cta",)]
-            ppc = min(kchunk, kres - q * kchunk) // 256
-            for ut in range(u_n):
-                lt = blk * bt + ut
-                has = lt < my_tiles
-                if ut + 1 < u_n and lt + 1 < my_tiles:
-                    nxt = lt + 1
-                elif q + 1 < n_chunks:
-                    nxt = blk * bt
-                else:
-                    nxt = (blk + 1) * bt
-                nxt_has = has and nxt < my_tiles
-                stage, parity = m_wait % stages, (m_wait // stages) & 1
-                if has:
-                    m_wait += 1
-                for p in range(ppc):
-                    if g == 0:
-                        if turn > 0:
-                            ops.append(("wait", 1))
-                    else:
-                        ops.append(("wait", 2))
-                    if p == 0 and has:
-                        if stages == 2 and nxt_has:
-                            ops.append(("issue", m_issue % 2, nxt))
-                            m_issue += 1
-                        ops.append(("consume", stage, parity, lt))
-                    last = p + 1 == ppc
-                    if g == 0:
-                        ops.append(("give", 2))
-                    elif turn + 1 < total_turns:
-                        ops.append(("give", 1))
-                    if stages == 1 and last and nxt_has:
-                        ops.append(("issue", 0, nxt))
-                        m_issue += 1
-                    if has:
-                        ops.append(("use", lt, q, p))
-                    turn += 1
+    for lt in range(steps):
+        has = lt < my_tiles
+        nxt_has = has and lt + 1 < my_tiles
+        stage, parity = lt % stages, (lt // stages) & 1
+        for p in range(passes):
+            if g == 0:
+                if turn > 0:
+                    ops.append(("wait", 1))
+            else:
+                ops.append(("wait", 2))
+            if p == 0 and has:
+                if stages == 2 and nxt_has:
+                    ops.append(("issue", (lt + 1) % 2, lt + 1))
+                ops.append(("consume", stage, parity, lt))
+            last = p + 1 == passes
+            if g == 0:
+                ops.append(("give", 2))
+            elif turn + 1 < total_turns:
+                ops.append(("give", 1))
+            if stages == 1 and last and nxt_has:
+                ops.append(("issue", 0, lt + 1))
+            if has:
+                ops.append(("use", lt, p))
+            turn += 1
     ops.append(("cta",))
     return ops
 
 
-def run_cta(n, grid, b, kres, kchunk, bt, stages):
-    progs = [group_program(g, n, grid, b, kres, kchunk, bt, stages) for g in range(2)]
+def run_cta(n, grid, b, kres, stages):
+    progs = [group_program(g, n, grid, b, kres, stages) for g in range(2)]
     pc = [0, 0]
     gives, waits = {1: 0, 2: 0}, {1: 0, 2: 0}
     arrived, blocked = [0, 0], [False, False]
@@ -127,20 +108,18 @@ def run_cta(n, grid, b, kres, kchunk, bt, stages):
     return used
 
 
-@pytest.mark.parametrize("kres,kchunk,bts", [(256, 256, [1]), (768, 768, [1]), (1024, 256, [8, 4]),
-                                             (1024, 512, [8, 3]), (1280, 512, [4])])
+@pytest.mark.parametrize("kres", [256, 512, 768, 1024])
 @pytest.mark.parametrize("stages", [1, 2])
 @pytest.mark.parametrize("n", [1, 63, 64, 65, 128, 129, 4097, 148 * 128 * 3 + 65])
-def test_resident_control_flow(n, stages, kres, kchunk, bts):
+def test_resident_control_flow(n, stages, kres):
     n_tiles = (n + R - 1) // R
     for grid_max in (148, 3):
         grid = min((n + 127) // 128, grid_max)
-        for bt in bts:
-            seen = {}
-            for b in range(grid):
-                used = run_cta(n, grid, b, kres, kchunk, bt, stages)
-                for g in range(2):
-                    for lt, q, p in used[g]:
-                        seen.setdefault(2 * (b + lt * grid) + g, []).append((q, p))
-            assert sorted(seen) == list(range(n_tiles))
-            assert all(len(v) == kres // 256 and len(set(v)) == len(v) for v in seen.values())
+        seen = {}
+        for b in range(grid):
+            used = run_cta(n, grid, b, kres, stages)
+            for g in range(2):
+                for lt, p in used[g]:
+                    seen.setdefault(2 * (b + lt * grid) + g, []).append(p)
+        assert sorted(seen) == list(range(n_tiles))
+        assert all(v == list(range(kres // 256)) for v in seen.values())
