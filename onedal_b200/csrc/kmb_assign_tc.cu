@@ -1492,8 +1492,7 @@ int launch_assign_tc(const void *Xhi, const void *Xlo, int64_t n, int64_t d, con
                                   : (bn == 256 ? tc::assign_tc_own_kernel<256, 3> : tc::assign_tc_own_kernel<128, 3>);
         if (allow_smem((const void *)kern) != cudaSuccess)
             return KMB_ECUDA;
-        const int grid = num_sms < 0 ? p.n_tiles : (int)std::min<int64_t>(num_sms, p.n_tiles);
-        kern<<<grid, tc::NTHREADS, smem, s>>>(mXh, mXl, mCh, mCl, p);
+        kern<<<std::min(num_sms, p.n_tiles), tc::NTHREADS, smem, s>>>(mXh, mXl, mCh, mCl, p);
         KMB_LAUNCHED();
         return cudaGetLastError() == cudaSuccess ? KMB_OK : KMB_ECUDA;
     }

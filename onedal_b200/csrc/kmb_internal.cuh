@@ -39,7 +39,7 @@ struct LoopState {
     int upd_mode;         // 0: recompute from all rows (counting sort), 1: apply the moved rows
     int upd_valid;        // sums, counts and previous labels describe the previous pass
     long long n_moved;    // rows whose label changed in this pass
-    double objective;     // the small train's exact objective (kmb_small.cu)
+    double objective;     // the exact objective of the call's last pass (train, infer, CSR)
 };
 
 // Grid-wide barrier of a cooperative launch: count and ticket are zero at its start.

@@ -12,7 +12,9 @@
 //   assign      one row per thread, the row's values in registers, the centroids broadcast
 //               from shared memory; the dot products add x_t * c_t in ascending t from
 //               zero with FMAs, norms and half norms are summed in the order of the
-//               separate kernels: the same scores, labels and distances bit for bit
+//               separate kernels: for floats, and for doubles with k <= 32, the same
+//               scores, labels and distances bit for bit (wider double problems are
+//               scored on the tensor pipe there, in its own order)
 //   accumulate  the CTA's rows are listed by label (stable); a thread per (segment of the
 //               list, column) sums its runs of equal labels, and a cluster's runs are
 //               added in order: float values as the exact integers of the exact update,
@@ -253,7 +255,6 @@ __device__ __forceinline__ void list_rows(const int *lab, int rows, int k, unsig
     const int tid = threadIdx.x, lane = tid & 31;
     const int nseg = min(32, kNT / k);  // k <= kSmallTrainMaxK <= kNT
     const int L = ((rows + nseg - 1) / nseg + 3) & ~3;  // rows per segment, whole int4s
-    const int users = min(kNT, k * nseg);
     // thread (segment s, cluster j) counts, then lists, its segment's rows of j
     const int j = tid % k, s = tid / k, e = min(rows, (s + 1) * L);
     const bool user = tid < k * nseg;
