@@ -1,6 +1,7 @@
-"""Small dense trains in one launch against the general path: the same problem, asked for
-with the FP64 recheck (which the general path alone takes) at values whose near ties are
-exact, so that both give the same responses. Sizes at the edges of the rule and of the
+"""Small dense trains in one launch against the general path, which a call takes while kernel
+timing is on (float: the same arithmetic, so everything is equal bit for bit) or with the
+FP64 recheck (double: at values whose near ties are exact, so that both give the same
+responses). Sizes at the edges of the rule and of the
 kernel: one CTA and many, ragged rows per CTA, the padded column counts, one cluster, as
 many clusters as threads allow, fewer rows than clusters would fill, empty clusters over
 several CTAs."""
@@ -42,17 +43,23 @@ def test_equals_the_general_path(dt, n, d, k, T, dup):
     desc = kmeans.descriptor(dt).set_cluster_count(k).set_max_iteration_count(T)
     desc.set_compute_form(kmeans.compute_form.plain)
     a = kmeans.train(desc, X, C0)
-    b = kmeans.train(desc.set_recheck(True), X, C0)
+    if dt == np.float32:
+        ctx = _native.context(0)
+        ctx.check(ctx.lib.kmb_context_set_kernel_timing(ctx.handle, 1))
+        try:
+            b = kmeans.train(desc, X, C0)
+        finally:
+            ctx.check(ctx.lib.kmb_context_set_kernel_timing(ctx.handle, 0))
+    else:
+        b = kmeans.train(desc.set_recheck(True), X, C0)
     assert a.get_iteration_count() == b.get_iteration_count()
     assert a.stats.empty_cluster_events == b.stats.empty_cluster_events
+    np.testing.assert_array_equal(a.get_responses(), b.get_responses())
     if dt == np.float32:
+        np.testing.assert_array_equal(a.get_model().get_centroids(), b.get_model().get_centroids())
         lab, _, _ = restated.assign_f32_in_f64(X, a.get_model().get_centroids())
-        same = (a.get_responses() == b.get_responses()).all()
-        if same:
-            np.testing.assert_array_equal(a.get_model().get_centroids(), b.get_model().get_centroids())
         assert (a.get_responses().ravel() == lab).mean() > 0.999
     else:
-        np.testing.assert_array_equal(a.get_responses(), b.get_responses())
         # sums in another order: n additions of values below M, 2^-53 each, over the count
         ca, cb = a.get_model().get_centroids(), b.get_model().get_centroids()
         np.testing.assert_allclose(ca, cb, rtol=0, atol=n * 2.0 ** -52 * np.abs(X).max())
