@@ -180,9 +180,17 @@ int serve_form(const Server *srv, const Model &m, int64_t n) {
 }
 
 size_t infer_bytes(int64_t n, int64_t d) { return (size_t)n * d * 4 + (size_t)n * 8 + (size_t)n * 4 + 4096; }
-size_t train_bytes(int64_t n, int64_t d, int64_t k) {
-    // rows + the context workspace of a small train (labels, sort buffers, records)
-    return (size_t)n * d * 4 + (size_t)n * 40 + (size_t)k * d * 64 + (size_t)(n / 512 + k) * d * 8 + (8u << 20);
+// The rows and the context workspace of a train: the one-launch form's scratch, or labels, sort
+// buffers and records (32 bytes a piece and column) of the separate kernels.
+size_t train_bytes(int64_t n, int64_t d, int64_t k, int device) {
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    const size_t rows = (size_t)n * d * 4, fixed = 8u << 20;
+    const kmb::SmallPlan small = kmb::make_small_plan<float>(n, d, k, sms);
+    if (small.ctas) return rows + (size_t)n * 4 + (size_t)k * d * 8 + kmb::small_scratch_bytes<float>(small, d, k) + fixed;
+    const kmb::UpdatePlan plan = kmb::make_update_plan(n, k, d);
+    return rows + (size_t)n * 40 + (size_t)k * d * 64 + (size_t)plan.max_pieces * d * 32 +
+           (size_t)plan.n_chunks * k * 4 + fixed;
 }
 
 void batch_done(Lane *lane) {
@@ -805,7 +813,7 @@ int kmb_server_submit_train(void *handle, const float *X_host, int64_t n, int64_
         r->C0 = C0_host;
         r->labels_out = labels_host;
         r->C_out = C_out_host;
-        r->bytes = train_bytes(n, d, k);
+        r->bytes = train_bytes(n, d, k, srv->device);
         r->t_submit = Clock::now();
         srv->all[r->id] = r;
         srv->train_queue.push_back(r);

@@ -131,6 +131,17 @@ def test_budget_is_respected_and_queued_requests_complete():
         assert st["in_use_bytes"] == 0
 
 
+def test_a_trains_workspace_counts_against_the_budget():
+    """A small train's device bytes: at least its rows and the blocks' sums, 24 bytes per
+    centroid value and block (92 of them)."""
+    n, d, k = 8_000, 60, 100
+    X = np.random.default_rng(35).standard_normal((n, d)).astype(np.float32)
+    with KMeansServer(hbm_budget_bytes=8 << 30, lanes=1, trainers=1) as srv:
+        before = srv.stats()["in_use_bytes"]
+        srv.wait(srv.submit_train(X, X[:k].copy(), 2), timeout=60)
+        assert srv.stats()["peak_in_use_bytes"] - before >= 4 * n * d + 24 * k * d * 92
+
+
 def test_submit_from_many_threads():
     rng = np.random.default_rng(33)
     C = rng.uniform(-1, 1, (200, 32)).astype(np.float32)
