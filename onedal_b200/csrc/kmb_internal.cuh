@@ -95,6 +95,21 @@ __device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived, long 
 // with less would refuse the launches of another that needs more.
 cudaError_t allow_smem(const void *kern);
 
+// Keys in the order of the values, for the choice of the farthest rows (32 bits of a float's, 64
+// of a double's). NaN has the smallest: the reference's candidate list takes no NaN over a
+// number. Said outright, since the bit operations alone may become floating-point ones, which
+// leave the bits of a NaN open.
+__device__ __forceinline__ unsigned long long order_key(float v) {
+    if (v != v) return 0;
+    const unsigned u = __float_as_uint(v);
+    return (u & 0x80000000u) ? (unsigned)~u : (u | 0x80000000u);
+}
+__device__ __forceinline__ unsigned long long order_key(double v) {
+    if (v != v) return 0;
+    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+    return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
+}
+
 // Recheck queue entry written by the assignment kernels for near-tie rows.
 struct RecheckEntry {
     int row;

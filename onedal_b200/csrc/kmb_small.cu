@@ -58,15 +58,6 @@ template <> struct Acc<double> {
 };
 template <typename F> constexpr int planes_of() { return (int)(sizeof(Acc<F>) / 8); }
 
-__device__ __forceinline__ unsigned long long key_of(float v) {
-    const unsigned u = __float_as_uint(v);
-    return (u & 0x80000000u) ? (unsigned)~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ unsigned long long key_of(double v) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
-    return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
-}
-
 struct SmallCand {
     unsigned long long key;
     long long row;
@@ -325,7 +316,7 @@ __device__ void farthest_rows(const F *d2, int rows, int have, int64_t row0, int
             bool in = r < rows;
             unsigned digit = 0;
             if (in) {
-                const unsigned long long key = key_of(d2[r]);
+                const unsigned long long key = order_key(d2[r]);
                 const unsigned inv = 0xffffu - (unsigned)r;
                 if (q < KD) {
                     in = ((key ^ key_low) >> ks) >> 8 == 0;
@@ -374,17 +365,17 @@ __device__ void farthest_rows(const F *d2, int rows, int have, int64_t row0, int
         if (s_all) break;  // (uniform; the next writes of s_* lie behind a barrier)
     }
     for (int r = tid; r < rows; r += kNT) {
-        const unsigned long long key = key_of(d2[r]);
+        const unsigned long long key = order_key(d2[r]);
         if (key > key_low || (key == key_low && 0xffffu - (unsigned)r >= row_low)) chosen[atomicAdd(&s_at, 1)] = r;
     }
     __syncthreads();
     for (int e = tid; e < have; e += kNT) {
         const int r = chosen[e];
-        const unsigned long long key = key_of(d2[r]);
+        const unsigned long long key = order_key(d2[r]);
         int rank = 0;
         for (int i = 0; i < have; ++i) {
             const int o = chosen[i];
-            const unsigned long long ok = key_of(d2[o]);
+            const unsigned long long ok = order_key(d2[o]);
             rank += ok > key || (ok == key && o < r);
         }
         out[rank] = SmallCand{key, (long long)(row0 + r)};

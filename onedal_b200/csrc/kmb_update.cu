@@ -367,24 +367,6 @@ __global__ void sums_kernel(const double *__restrict__ records, const int64_t *_
 
 // ---- empty-cluster reseeding: top-m rows by squared distance ---------------
 
-template <typename F> struct KeyOf;
-template <> struct KeyOf<float> {
-    using U = unsigned int;
-    static constexpr int BITS = 32;
-    __device__ static U key(float v) {
-        const U u = __float_as_uint(v);
-        return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-    }
-};
-template <> struct KeyOf<double> {
-    using U = unsigned long long;
-    static constexpr int BITS = 64;
-    __device__ static U key(double v) {
-        const U u = (U)__double_as_longlong(v);
-        return (u & 0x8000000000000000ull) ? ~u : (u | 0x8000000000000000ull);
-    }
-};
-
 constexpr int kTailThreads = 512;
 constexpr int kTailWarps = kTailThreads / 32;
 constexpr int kSelBits = 11;               // radix-select digit
@@ -444,7 +426,6 @@ __device__ void cand_sort(Cand *buf, int P) {
 template <typename F>
 __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync *sy, unsigned &arrived, long long wait,
                            Cand *__restrict__ cand) {
-    using K = KeyOf<F>;
     __shared__ unsigned s_hist[kSelBins];
     __shared__ unsigned s_scan[kTailWarps];
     __shared__ int s_digit;
@@ -456,7 +437,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
     unsigned long long prefix = 0, mask = 0;
     unsigned need = (unsigned)m, eq_total = 0;
     int round = 0;
-    for (int top = K::BITS; top > 0; ++round) {
+    for (int top = 8 * (int)sizeof(F); top > 0; ++round) {
         const int bits = min(kSelBits, top);
         const int shift = top - bits;
         for (int i = tid; i < kSelBins; i += kTailThreads) s_hist[i] = 0;
@@ -470,7 +451,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
 #pragma unroll
             for (int q = 0; q < 8; ++q) {
                 if (i + q * stride >= n) continue;
-                const unsigned long long key = (unsigned long long)K::key(v[q]);
+                const unsigned long long key = order_key(v[q]);
                 if ((key & mask) == prefix) atomicAdd(&s_hist[(unsigned)(key >> shift) & dmask], 1u);
             }
         }
@@ -524,7 +505,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             if (i + q * stride >= n) continue;
-            const unsigned long long key = (unsigned long long)K::key(v[q]);
+            const unsigned long long key = order_key(v[q]);
             if (key > prefix || (all_eq && key == prefix)) {
                 const unsigned at = atomicAdd(&sy->n_cand, 1u);
                 if (at < (unsigned)m) cand[at] = Cand{key, (long long)(i + q * stride)};
@@ -550,7 +531,7 @@ __device__ bool select_top(const F *__restrict__ d2, int64_t n, int m, TailSync 
                 const unsigned base = s_base;
                 if (base >= (unsigned)m) break;
                 const int64_t i = b0 + tid;
-                const bool eq = i < n && (unsigned long long)K::key(__ldcg(d2 + i)) == prefix;
+                const bool eq = i < n && order_key(__ldcg(d2 + i)) == prefix;
                 const unsigned votes = __ballot_sync(0xffffffffu, eq);
                 if (lane == 0) s_scan[warp] = (unsigned)__popc(votes);
                 __syncthreads();

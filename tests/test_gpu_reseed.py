@@ -9,12 +9,12 @@ import numpy as np
 import pytest
 import torch
 
-from onedal_b200 import _native
+from onedal_b200 import _native, kmeans
 
 pytestmark = pytest.mark.gpu
 
 
-def _step(X, C):
+def _step(X, C, form=_native.KMB_FORM_PLAIN):
     ctx = _native.context(0)
     n, d = X.shape
     Xd, Cd = torch.from_numpy(X).cuda(), torch.from_numpy(C).cuda()
@@ -23,7 +23,7 @@ def _step(X, C):
     ctx.set_stream(torch.cuda.current_stream().cuda_stream)
     dtype = _native.KMB_F32 if X.dtype == np.float32 else _native.KMB_F64
     ctx.check(ctx.lib.kmb_lloyd_step(ctx.handle, dtype, Xd.data_ptr(), n, d, Cd.data_ptr(), C.shape[0],
-                                     _native.KMB_FORM_PLAIN, 0, out.data_ptr(), lab.data_ptr(), ctypes.byref(shift),
+                                     form, 0, out.data_ptr(), lab.data_ptr(), ctypes.byref(shift),
                                      ctypes.byref(ne)))
     return out.cpu().numpy(), lab.cpu().numpy(), ne.value
 
@@ -59,3 +59,26 @@ def test_one_blocks_sort_outlasts_a_wait(monkeypatch):
     assert ne == m and (lab == 0).all()
     order = np.lexsort((np.arange(n), -(X.astype(np.int64) ** 2).sum(1)))[:m]
     np.testing.assert_array_equal(out[1:], X[order])
+
+
+@pytest.mark.parametrize("n,m", [(40, 39), (300, 5), (5000, 60), (70_000, 300)])
+@pytest.mark.parametrize("dt,form", [(np.float32, _native.KMB_FORM_PLAIN), (np.float64, _native.KMB_FORM_PLAIN),
+                                     (np.float32, _native.KMB_FORM_BF16X3)])
+def test_rows_with_a_nan_come_last(dt, form, n, m):
+    """A NaN row's distance is no number: it reseeds a cluster only when no other row is left, in
+    an update of the separate kernels and in a small train."""
+    d = 5
+    rng = np.random.default_rng(n)
+    X = rng.integers(-100, 101, (n, d)).astype(dt)
+    nan_rows = np.array([0, 7, n // 2, n - 1])
+    X[nan_rows, [0, 1, 2, 3]] = np.array([1, -1, 1, -1]) * np.nan
+    C = np.full((m + 1, d), 10000, dt)
+    C[0] = 0
+    dist = (X.astype(np.float64) ** 2).sum(1)
+    order = np.lexsort((np.arange(n), -np.where(np.isnan(dist), -1, dist)))[:m]
+    out, lab, ne = _step(X, C, form)
+    assert ne == m and (lab == 0).all()
+    np.testing.assert_array_equal(out[1:], X[order])
+    if form == _native.KMB_FORM_PLAIN and m < 256:
+        desc = kmeans.descriptor(dt).set_cluster_count(m + 1).set_max_iteration_count(1).set_compute_form(form)
+        np.testing.assert_array_equal(kmeans.train(desc, X, C).get_model().get_centroids()[1:], X[order])
