@@ -37,6 +37,7 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <type_traits>
 
 namespace kmb {
 namespace {
@@ -490,7 +491,6 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
     // the finalize takes 2^lg lanes a cell: as many as there are CTAs, a warp at most
     int lg = 0;
     while (lg < 5 && 1 << lg < G) ++lg;
-    const int sub = lane & ((1 << lg) - 1), slot = lane >> lg;
     while (ok && !done && iterations < a.T) {
         assign_rows<F, DMAX>(Xs, ds, Cs, hs, xn, rows, d, k, lab, d2);
         __syncthreads();
@@ -565,46 +565,52 @@ __global__ void __launch_bounds__(kNT, 1) small_train_kernel(const SmallArgs<F> 
         if (!(ok = grid_sync(sync, arrived, a.wait))) break;
         // finalize over the grid (256 x 64, k = 256, one CTA: 1460 us a train with a warp per
         // cell, 235 us with a thread)
-        for (int first = (b * kNW + warp) << (5 - lg); first < cells; first += (G * kNW) << (5 - lg)) {
-            const int cell = first + slot;
-            const bool in = cell < cells;
-            const int j = in ? cell / d : 0, t = in ? cell - j * d : 0;
-            Acc<F> s = {};
-            int cnt = 0;
-            for (int c0 = sub; c0 < G; c0 += 5 * 32) {  // five CTAs' loads in flight per lane
-                unsigned long long v[5][NP];
-                int n5[5];
+        auto finalize = [&](auto whole) {  // whole: a warp a cell, known at compile time
+            constexpr bool W = decltype(whole)::value;
+            const int per = W ? 1 : 32 >> lg, sub = W ? lane : lane & ((1 << lg) - 1);
+            for (int first = (b * kNW + warp) * per; first < cells; first += G * kNW * per) {
+                const int cell = W ? first : first + (lane >> lg);
+                const bool in = W || cell < cells;
+                const int j = in ? cell / d : 0, t = in ? cell - j * d : 0;
+                Acc<F> s = {};
+                int cnt = 0;
+                for (int c0 = sub; c0 < G; c0 += 5 * 32) {  // five CTAs' loads in flight per lane
+                    unsigned long long v[5][NP];
+                    int n5[5];
 #pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    const int c = c0 + 32 * q;
-                    n5[q] = in && c < G ? __ldcg(a.part_cnt + (size_t)j * G + c) : 0;
+                    for (int q = 0; q < 5; ++q) {
+                        const int c = c0 + 32 * q;
+                        n5[q] = in && c < G ? __ldcg(a.part_cnt + (size_t)j * G + c) : 0;
 #pragma unroll
-                    for (int l = 0; l < NP; ++l)
-                        v[q][l] = in && c < G ? __ldcg(a.part + ((size_t)l * cells + cell) * G + c) : 0ull;  // (0.0 too)
+                        for (int l = 0; l < NP; ++l)
+                            v[q][l] = in && c < G ? __ldcg(a.part + ((size_t)l * cells + cell) * G + c) : 0ull;  // (0.0 too)
+                    }
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) {
+                        cnt += n5[q];
+#pragma unroll
+                        for (int l = 0; l < NP; ++l) s.v[l] += *reinterpret_cast<const decltype(s.v[0] + 0) *>(&v[q][l]);
+                    }
                 }
 #pragma unroll
-                for (int q = 0; q < 5; ++q) {
-                    cnt += n5[q];
+                for (int m = 16; m >= 1; m >>= 1) {
+                    if (!W && m >> lg) continue;
 #pragma unroll
-                    for (int l = 0; l < NP; ++l) s.v[l] += *reinterpret_cast<const decltype(s.v[0] + 0) *>(&v[q][l]);
+                    for (int l = 0; l < NP; ++l) s.v[l] += __shfl_xor_sync(0xffffffffu, s.v[l], m);
+                    cnt += __shfl_xor_sync(0xffffffffu, cnt, m);
+                }
+                if (in && sub == 0) {
+                    const F old = Cs[j * DMAX + t];
+                    const F c = cnt > 0 ? centroid_of(s, sizeof(F) == 4 ? s_exp[t] : 0, cnt) : old;
+                    const double df = (double)old - (double)c;
+                    a.C_new[cell] = c;
+                    a.dshift[cell] = cnt > 0 ? df * df : 0.0;
+                    if (t == 0) a.counts[j] = cnt;
                 }
             }
-#pragma unroll
-            for (int m = 16; m >= 1; m >>= 1) {
-                if (m >> lg) continue;
-#pragma unroll
-                for (int l = 0; l < NP; ++l) s.v[l] += __shfl_xor_sync(0xffffffffu, s.v[l], m);
-                cnt += __shfl_xor_sync(0xffffffffu, cnt, m);
-            }
-            if (in && sub == 0) {
-                const F old = Cs[j * DMAX + t];
-                const F c = cnt > 0 ? centroid_of(s, sizeof(F) == 4 ? s_exp[t] : 0, cnt) : old;
-                const double df = (double)old - (double)c;
-                a.C_new[cell] = c;
-                a.dshift[cell] = cnt > 0 ? df * df : 0.0;
-                if (t == 0) a.counts[j] = cnt;
-            }
-        }
+        };
+        if (lg == 5) finalize(std::true_type());
+        else finalize(std::false_type());
         if (!(ok = grid_sync(sync, arrived, a.wait))) break;
         // every CTA: the new centroids, the shift, the empty clusters
         double part = 0.0;
