@@ -109,14 +109,13 @@ def test_threads_get_what_they_get_alone(make):
 
 @pytest.mark.parametrize("n", [100, 2000], ids=["one_block", "blocks"])
 def test_a_small_train_does_not_wait_for_another_threads(n):
-    """A train of eight blocks that never converges (a NaN in its rows) runs for its 20,000
-    iterations; a thread with a few blocks' train, which the other SMs can hold, is done long
-    before."""
+    """A train of eight blocks that never converges (a NaN in doubles makes every shift a NaN)
+    runs for its 25,000 iterations; a thread with a few blocks' train, which the other SMs can
+    hold, is done long before."""
     def args(n, T):
-        X, C = _rows(n, 20, 20)
-        desc = kmeans.descriptor(np.float32).set_cluster_count(20).set_max_iteration_count(T)
-        return desc.set_compute_form(kmeans.compute_form.plain), X, C
-    long_args, short_args = args(2001, 20_000), args(n, 3)
+        X, C = (t.double() for t in _rows(n, 20, 20))
+        return kmeans.descriptor(np.float64).set_cluster_count(20).set_max_iteration_count(T), X, C
+    long_args, short_args = args(2001, 25_000), args(n, 3)
     long_args[1][5, 5] = float("nan")
     kmeans.train(*short_args)
     ended = {}
