@@ -96,8 +96,8 @@ __device__ __forceinline__ bool grid_sync(GridSync *sy, unsigned &arrived, long 
 cudaError_t allow_smem(const void *kern);
 
 // Keys in the order of the values, for the choice of the farthest rows (32 bits of a float's, 64
-// of a double's). NaN has the smallest: the reference's candidate list takes no NaN over a
-// number. Said outright, since the bit operations alone may become floating-point ones, which
+// of a double's). NaN has the smallest: the reference's candidate list, once it is full, takes
+// none. Said outright, since the bit operations alone may become floating-point ones, which
 // leave the bits of a NaN open.
 __device__ __forceinline__ unsigned long long order_key(float v) {
     if (v != v) return 0;
